@@ -83,6 +83,10 @@ struct DetTileArgs {               // noise-off DP step over 64 x 32 tiles of ev
 // launchers (defined in the kernel translation units)
 template <typename T>
 cudaError_t launch_dornic(const DornicArgs<T>& a, int rem, int grid, int block, cudaStream_t s);
+template <>   // tm_step.cu
+cudaError_t launch_dornic<float>(const DornicArgs<float>& a, int rem, int grid, int block, cudaStream_t s);
+template <>   // tm_step64.cu
+cudaError_t launch_dornic<double>(const DornicArgs<double>& a, int rem, int grid, int block, cudaStream_t s);
 template <typename T>
 cudaError_t launch_rk4(const RK4Args<T>& a, bool det, int grid, cudaStream_t s);
 template <typename T>

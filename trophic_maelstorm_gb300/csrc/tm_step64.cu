@@ -1,0 +1,605 @@
+// tm_step64.cu -- the fused Dornic step in FP64.
+//
+// The step is the one of tm_step.cu: the same streams, the same operations in the
+// same order, the same bits.  What differs is what GB300 does cheaply.  One FP64
+// warp instruction occupies its scheduler's FP64 pipe for 64-76 cycles, however
+// many lanes it has, so the kernel is written around how few of them a site needs:
+//   * absorbing sites are found by the bits of the five values (row masks from
+//     ballots), without an FP64 operation;
+//   * the Poisson search, the squeeze, the ziggurat's wedge test and the log test
+//     only decide something.  They run in FP32 with an error bound, and the FP32
+//     answer is taken where the bound proves that the FP64 comparison has the same
+//     outcome; the rest (0.1-0.2 % of the searches) do the FP64 comparison;
+//   * divisions, square roots and some products are rounded exactly on the integer
+//     pipe (tm_f64.cuh).
+// The whole warp runs the straight-line draw together (lanes without a site repeat
+// one): lanes that left the search one by one made the rest of the draw run twice.
+// Measured, 16 lattices of 256^2, 32 steps of a decaying run: RK4 remainder 20.2 ->
+// 4.4 ms; general sampler for every site 319 FP64 instructions per 32 sites, now about 30
+// (Euler-exact remainder).  Bound by the FP64 pipe (60-65 % busy) and the integer
+// pipe together.  Two CTAs of 8 warps per SM: three (80 registers, small spills) took
+// the same time, four 13 % more.
+//
+// Sites the straight-line draw cannot finish are carried in three lists per warp
+// and drawn 32 at a time, so that a rare path runs with full lanes: the whole
+// general sampler (list 0), the general Gamma draw with its shape known (list 1)
+// and the boost U^(1/k) of shapes below 1 (list 2).  A draw depends only on (seed,
+// site, step), so it may run in any later pass of the same warp.
+#include "tm_device.cuh"
+#include "tm_kernels.cuh"
+
+namespace tmg {
+
+namespace {
+
+constexpr int kWarps = 8;
+constexpr int kSearch = 96;                 // terms of the FP32 Poisson search (multiple of 4)
+constexpr int kListCap = 64;                // carried entries of one list: up to 31, and 32 new ones
+
+struct Tab64 : SmemTab<double> {
+    __align__(16) float rcpf[kSearch + 8];  // rcpf[3 + n] = 1/n: the search reads n = 4 i + 1 .. 4 i + 4 at once
+    __device__ __forceinline__ void fill_all()
+    {
+        fill();
+        for (int i = threadIdx.x; i < kSearch + 8; i += blockDim.x) rcpf[i] = i > 3 ? 1.0f / (float)(i - 3) : 0.0f;
+    }
+};
+
+struct ListEntry {                          // 24 bytes
+    int k;                                  // instance
+    uint32_t site;
+    double a, b;
+};
+
+__host__ __device__ __forceinline__ size_t warp_bytes(int rows_cap)
+{
+    return 3 * kListCap * sizeof(ListEntry) + (size_t)rows_cap * 32 * sizeof(unsigned short);
+}
+
+// h w of a ziggurat value h (below 2^24) and its layer's width, rounded once
+__device__ __forceinline__ double signed_mul(int32_t h, double w)
+{
+    return tmf::with_sign(tmf::from_u31((uint32_t)(h < 0 ? -h : h)), h < 0) * w;
+}
+
+__device__ __forceinline__ uint32_t hi32(double x) { return (uint32_t)__double2hiint(x); }
+
+// Upper bound of |FP32 search's tail - FP64 search's tail| for a mean below 32.
+// The rounding of m (relative 2^-23) moves a tail by at most m 2^-23 max p <= 0.4
+// m 2^-23; a term p_i carries 3 i + 4 roundings, which sum to (3 m + 4) 2^-24, and the
+// differences q - p another m 2^-24: (4 m + 8) 2^-24 in all.  The largest
+// difference seen over 3 10^6 means is a fifth of this bound.
+__device__ __forceinline__ float search_eps(float m) { return (m + 4.0f) * 0x1p-22f; }
+
+// Poisson count for the mean m < 32 and the 32-bit uniform w of the lanes with
+// `need`, by the search of poisson_exact in FP32; -1 where a tail lies within the
+// bound of u.  The whole warp runs it: lanes that leave a search loop one by one
+// would drag the rest of the draw through the pipe in pieces.
+__device__ __forceinline__ int search_count(bool need, float m, uint32_t w, const float* rcp)
+{
+    const float eps = search_eps(m);
+    const float u = (float)w * 0x1p-32f;
+    const float up = u + eps, dn = u - eps;
+    float p = tm_exp_neg_small(-m);
+    float q = (m < 0.25f) ? tm_negexpm1(m) : 1.0f - p;
+    bool run = need && up < q;
+    int n = q <= dn ? 0 : -1;
+    for (int it = 0; it < kSearch && __any_sync(0xffffffffu, run); it += 4) {
+        // four terms per trip; the tails only decrease, so those certainly above u form a prefix
+        const float4 r4 = *reinterpret_cast<const float4*>(rcp + it + 1);
+        const float p1 = (p * m) * r4.x, q1 = q - p1;
+        const float p2 = (p1 * m) * r4.y, q2 = q1 - p2;
+        const float p3 = (p2 * m) * r4.z, q3 = q2 - p3;
+        p = (p3 * m) * r4.w;
+        q = q3 - p;
+        const bool a1 = up < q1, a2 = up < q2, a3 = up < q3;
+        const float first = a2 ? (a3 ? q : q3) : (a1 ? q2 : q1);     // the first tail not certainly above u
+        const int c = a2 ? (a3 ? 4 : 3) : (a1 ? 2 : 1);
+        if (run && !(up < q)) {
+            n = first <= dn ? it + c : -1;
+            run = false;
+        }
+    }
+    return run ? -1 : n;
+}
+
+// FP32 value of a uniform from its two words, relative error 2^-22
+__device__ __forceinline__ float unit_f32(uint32_t w1, uint32_t w2)
+{
+    return fmaf((float)w1, 0x1p-32f, (float)((w2 >> 11) + 1u) * 0x1p-53f);
+}
+
+// Stream<double>::normal with the wedge test decided in FP32 where its error
+// (below 2^-20 on values up to 1) allows.
+template <int CAP>
+__device__ __forceinline__ double normal64(Stream<double>& g, const Tab64& tb)
+{
+    for (int it = 0; it < CAP; ++it) {
+        const uint32_t w = g.u32();
+        const int iz = zig_layer(w);
+        const int32_t hz = zig_value(w);
+        const uint32_t az = (uint32_t)(hz < 0 ? -hz : hz);
+        const ZigLayer<double> zl = tb.zig[iz];
+        const double x = signed_mul(hz, zl.w);
+        if (az < zl.k) return x;
+        if (iz == 0) {
+            for (int jt = 0; jt < CAP; ++jt) {
+                const double xt = -tm_log_pos(g.open()) * (1.0 / kZigR);
+                const double yt = -tm_log_pos(g.open());
+                if (yt + yt >= xt * xt) {
+                    const double r = kZigR + xt;
+                    return hz < 0 ? -r : r;
+                }
+            }
+            break;
+        }
+        const double fb = tb.zf[iz], ft = tb.zf[iz + 1];
+        const double u = g.open();
+        const float xf = (float)x;
+        const float lhs = (float)fb + (float)u * ((float)ft - (float)fb);
+        const float diff = tm_exp(-0.5f * (xf * xf)) - lhs;
+        if (diff > 0x1p-18f) return x;
+        if (diff < -0x1p-18f) continue;
+        if (fb + u * (ft - fb) < tm_exp(-0.5 * (x * x))) return x;
+    }
+    g.status |= TM_STATUS_CAP_BIT;
+    return 0.0;
+}
+
+// gamma_mt with its two acceptance tests decided in FP32 where their error bounds
+// allow.
+template <int CAP>
+__device__ __forceinline__ double gamma64(Stream<double>& g, double k, const Tab64& tb)
+{
+    if (!(k > 0.0)) return 0.0;
+    const double kk = (k < 1.0) ? k + 1.0 : k;
+    const double d = kk - 1.0 / 3.0;
+    const double c = Tr<double>::inv_sqrt(9.0 * d);
+    double res = kk;
+    bool done = false;
+    for (int it = 0; it < CAP && !done; ++it) {
+        double x = 0.0, v = 0.0;
+        bool ok = false;
+        for (int jt = 0; jt < CAP; ++jt) {
+            x = normal64<CAP>(g, tb);
+            v = 1.0 + c * x;
+            if (v > 0.0) { ok = true; break; }
+        }
+        if (!ok) break;
+        const double mm = (v < 1.0) ? v : 1.0;
+        v = (v * v) * v;
+        const double u = g.open();
+        const float xf = (float)x, df = (float)d, vf = (float)v, uf = (float)u;
+        const float x2f = xf * xf;
+        if (vf > 1e-30f && uf < 0.999f && df < 1e6f) {
+            // squeeze: relative error of either side below 2^-20 (1 - u from u < 0.999: 2^-14)
+            const float lhs = (1.0f - uf) * ((108.0f * df) * (float)mm), rhs = x2f * x2f;
+            if (lhs > rhs * 1.001f) { res = d * v; done = true; break; }
+            // log test: absolute error below the margin
+            const float lu = tm_log_pos(uf), lv = tm_log_pos(vf);
+            const float margin = 0x1p-18f * ((2.0f + fabsf(lu)) + x2f + df * ((1.0f + vf) + fabsf(lv)));
+            const float gap = (0.5f * x2f + df * ((1.0f - vf) + lv)) - lu;
+            if (lhs < rhs * 0.999f) {
+                if (gap > margin) { res = d * v; done = true; break; }
+                if (gap < -margin) continue;
+            } else if (gap > margin) {      // either test accepts
+                res = d * v; done = true; break;
+            }
+        }
+        const double x2 = x * x;
+        if ((1.0 - u) * ((108.0 * d) * mm) > x2 * x2) { res = d * v; done = true; break; }
+        if (tm_log_pos(u) < 0.5 * x2 + d * ((1.0 - v) + tm_log(v))) { res = d * v; done = true; break; }
+    }
+    if (!done) g.status |= TM_STATUS_CAP_BIT;
+    if (k < 1.0) {
+        const double u = g.open();
+        res = res * tm_exp(tmf::div(tm_log_pos(u), k));
+    }
+    return res;
+}
+
+// -b x^2 (- c x^3)
+template <bool CUBIC>
+__device__ __forceinline__ double rem_f64(double x, double b, double c)
+{
+    double f = tmf::mul((-b) * x, x);
+    if (CUBIC) f = f - tmf::mul(tmf::mul(c * x, x), x);
+    return f;
+}
+template <bool CUBIC>
+__device__ __forceinline__ double rem_rk4(const DornicArgs<double>& A, double rs, double bi)
+{
+    const double k1 = rem_f64<CUBIC>(rs, bi, A.c);
+    const double k2 = rem_f64<CUBIC>(rs + A.dt2 * k1, bi, A.c);
+    const double k3 = rem_f64<CUBIC>(rs + A.dt2 * k2, bi, A.c);
+    const double k4 = rem_f64<CUBIC>(rs + A.dt * k3, bi, A.c);
+    return rs + A.dt6 * (fma(2.0, k3, fma(2.0, k2, k1)) + k4);
+}
+
+// Remainder, clamp and status bits of one site after its draw (finish_site of
+// tm_step.cu, with the comparisons on bits).
+template <int REM>
+__device__ __forceinline__ double finish64(const DornicArgs<double>& A, double rs, double bi, unsigned& st)
+{
+    double res;
+    if (REM == 0) {
+        res = tmf::div(rs, 1.0 + (bi * rs) * A.dt);
+    } else if (REM == 1) {
+        res = A.cubic ? rem_rk4<true>(A, rs, bi) : rem_rk4<false>(A, rs, bi);
+    } else {
+        res = rs;
+    }
+    if (REM != 2) {
+        // not below ceps if positive with larger bits (a NaN neither)
+        const long long rb = __double_as_longlong(res);
+        if (!(rb >= 0 && rb >= __double_as_longlong(A.ceps)) && rb != 0) {
+            if (tmf::hw_in_range(res, A.clo, A.ceps)) res = 0.0;
+        }
+        st |= value_status(res);
+    }
+    return res;
+}
+
+struct SiteMean {
+    double cur, alpha, m, mu1;
+};
+
+// Value, neighbour coupling, Poisson mean and Gamma shape of a site.
+__device__ __forceinline__ SiteMean site_mean(const DornicArgs<double>& A, const double* __restrict__ src, int L, int y,
+                                              int x, double pm)
+{
+    const int yn = (y == 0) ? L - 1 : y - 1, ys = (y == L - 1) ? 0 : y + 1;
+    const int xw = (x == 0) ? L - 1 : x - 1, xe = (x == L - 1) ? 0 : x + 1;
+    SiteMean s;
+    s.cur = src[(long long)y * L + x];
+    const double n = src[(long long)yn * L + x], so = src[(long long)ys * L + x];
+    const double w = src[(long long)y * L + xw], e = src[(long long)y * L + xe];
+    s.alpha = A.dcoef * (((n + so) + w) + e);
+    s.m = tmf::mul(pm, s.cur);
+    s.mu1 = tmf::mul(s.alpha, A.two_s2);
+    return s;
+}
+
+// Finish a drawn site and store it.
+template <int REM>
+__device__ __forceinline__ void store_site(const DornicArgs<double>& A, int k, uint32_t site, double rs, unsigned st)
+{
+    const long long o = A.it.off[k] + (long long)site;
+    double res = rs;
+    if (!(A.zero_fixed && __double_as_longlong(rs) == 0))
+        res = finish64<REM>(A, rs, A.site_b ? A.site_b[o] : A.b, st);
+    A.out[o] = res;
+    if (st) atomicOr(A.it.status + k, st);
+}
+
+// One carried entry of list `which`.
+template <int REM, int SAMP, int CAP>
+__device__ __forceinline__ void draw_general(const DornicArgs<double>& A, const Tab64& tab, long long step, bool whole,
+                                             const ListEntry& e)
+{
+    Stream<double> g;
+    g.init(A.it.seed[e.k], e.site, step);
+    double k = e.a;
+    bool gauss = false;
+    if (whole) {
+        const int L = A.it.L[e.k];
+        const int y = (int)(e.site / (uint32_t)L), x = (int)(e.site - (uint32_t)y * (uint32_t)L);
+        const SiteMean s = site_mean(A, A.in + A.it.off[e.k], L, y, x, A.it.consts[e.k].x);
+        double n = 0.0;
+        if (s.m > 0.0) {
+            if (SAMP == 1 && s.m > 100.0) {
+                const double z = normal64<CAP>(g, tab);
+                n = trunc(z * tmf::sqrt(s.m) + s.m);
+            } else {
+                n = poisson_exact<CAP>(g, s.m, (const SmemTab<double>&)tab);
+            }
+        }
+        k = s.mu1 + n;
+        gauss = SAMP == 1 && k > 100.0;
+    } else if (e.b != 0.0) {
+        (void)g.u32();                       // the word the count took
+    }
+    double gv;
+    if (gauss) {
+        const double z = normal64<CAP>(g, tab);
+        gv = z * tmf::sqrt(k) + k;
+    } else {
+        gv = gamma64<CAP>(g, k, tab);
+    }
+    store_site<REM>(A, e.k, e.site, gv * A.it.consts[e.k].y, g.status);
+}
+
+// The boost of a shape below 1: entry a = shape, b = the Gamma(shape + 1) draw,
+// negative where the site took no Poisson word.
+template <int REM>
+__device__ __forceinline__ void draw_boost(const DornicArgs<double>& A, long long step, const ListEntry& e)
+{
+    const unsigned long long seed = A.it.seed[e.k];
+    const uint32_t slo = (uint32_t)(unsigned long long)step, shi = (uint32_t)((unsigned long long)step >> 32);
+    const bool drew = (int32_t)hi32(e.b) >= 0;
+    const U4 r1 = philox4x32_10(e.site, slo, 1u, shi, (uint32_t)seed, (uint32_t)(seed >> 32));
+    uint32_t w1 = r1.x, w2 = r1.y;
+    if (!drew) {
+        const U4 r0 = philox4x32_10(e.site, slo, 0u, shi, (uint32_t)seed, (uint32_t)(seed >> 32));
+        w1 = r0.w;
+        w2 = r1.x;
+    }
+    const double u = tmf::open_unit(((unsigned long long)w1 << 21) | (unsigned long long)(w2 >> 11));
+    const double res = tmf::abs_bits(e.b) * tm_exp(tmf::div(tm_log_pos(u), e.a));
+    store_site<REM>(A, e.k, e.site, res * A.it.consts[e.k].y, 0u);
+}
+
+}  // namespace
+
+template <int REM, int SAMP, int CAP>
+__global__ void __launch_bounds__(256, 2) dornic_step64_kernel(const DornicArgs<double> A)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ Tab64 tab;
+    __shared__ int left[kWarps][3];
+    tab.fill_all();
+    __syncthreads();
+    const int warp = threadIdx.x >> 5;
+    unsigned char* const wbase = smem_raw + warp * warp_bytes(A.rows_cap);
+    ListEntry* const lists = reinterpret_cast<ListEntry*>(wbase);
+    unsigned short* const Wq = reinterpret_cast<unsigned short*>(lists + 3 * kListCap);
+    const int lane = threadIdx.x & 31;
+    const unsigned lt_mask = (1u << lane) - 1u;
+    // consecutive tasks go to different blocks, so that few tasks still spread over the SMs
+    const int gw = warp * (int)gridDim.x + (int)blockIdx.x;
+    const int nw = (int)gridDim.x * kWarps;
+    const long long step = (A.step_base ? *A.step_base : 0LL) + A.step_off;
+    int cnt[3] = {0, 0, 0};
+    // one more trip after the last task empties the lists of the whole block together
+    for (int t = gw;; t += nw) {
+        const bool more = t < A.n_tasks;
+        int k = 0, L = 0, x0 = 0, y0 = 0, nq = 0;
+        if (more) k = A.tasks[t].x;
+        if (more && (A.it.alive == nullptr || A.it.alive[k] != 0)) {
+            const int4 tk = A.tasks[t];
+            L = A.it.L[k];
+            const double* __restrict__ src = A.in + A.it.off[k];
+            x0 = tk.y;
+            y0 = tk.z;
+            const int rows = tk.w;
+            const int w = min(32, L - x0);
+            const int x = x0 + lane;
+            const bool act = lane < w;
+            // pass 1: a site is absorbing when it and its neighbours are zero, which row
+            // masks of non-zero values tell; absorbing sites are finished here
+            const bool erow = lane < rows;
+            const int xw = (x0 == 0) ? L - 1 : x0 - 1;
+            const int xe = (x0 + w == L) ? 0 : x0 + w;
+            const unsigned wm =
+                __ballot_sync(0xffffffffu, erow && !tmf::is_zero(erow ? src[(long long)(y0 + lane) * L + xw] : 0.0));
+            const unsigned em =
+                __ballot_sync(0xffffffffu, erow && !tmf::is_zero(erow ? src[(long long)(y0 + lane) * L + xe] : 0.0));
+            const int yn = (y0 == 0) ? L - 1 : y0 - 1;
+            const unsigned actm = __ballot_sync(0xffffffffu, act);
+            unsigned mn = __ballot_sync(0xffffffffu, act && !tmf::is_zero(act ? src[(long long)yn * L + x] : 0.0));
+            unsigned mc = __ballot_sync(0xffffffffu, act && !tmf::is_zero(act ? src[(long long)y0 * L + x] : 0.0));
+            unsigned st = 0;
+            for (int r0 = 0; r0 < rows; r0 += 8) {
+                double v[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    int y = y0 + r0 + j + 1;
+                    if (y >= L) y -= L;
+                    v[j] = (act && r0 + j < rows) ? src[(long long)y * L + x] : 0.0;
+                }
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const int r = r0 + j;
+                    if (r >= rows) break;
+                    const unsigned ms = __ballot_sync(0xffffffffu, !tmf::is_zero(v[j]));
+                    unsigned lm = mn | mc | ms | (mc << 1) | (mc >> 1) | ((wm >> r) & 1u) | (((em >> r) & 1u) << (w - 1));
+                    if (SAMP == 2) lm = 0xffffffffu;
+                    lm &= actm;
+                    if ((lm >> lane) & 1u) {
+                        Wq[nq + __popc(lm & lt_mask)] = (unsigned short)(r * 32 + lane);
+                    } else if (act) {
+                        const long long o = A.it.off[k] + (long long)(y0 + r) * L + x;
+                        double res = 0.0;
+                        if (!A.zero_fixed) res = finish64<REM>(A, 0.0, A.site_b ? A.site_b[o] : A.b, st);
+                        A.out[o] = res;
+                    }
+                    nq += __popc(lm);
+                    mn = mc;
+                    mc = ms;
+                }
+            }
+            if (st) atomicOr(A.it.status + k, st);
+            __syncwarp();
+        }
+        const unsigned long long seed = A.it.seed[k];
+        const Dc4 cs = A.it.consts[k];
+        // pass 2: the queued sites, 32 at a time, straight line and with the whole warp
+        // (lanes without a site draw the last one again); then whatever list is full
+        int base = 0;
+        do {
+            int outcome = -1;                  // -1 done, 0..2: the list that draws it
+            ListEntry en;
+            en.k = k;
+            if (base < nq) {
+                const bool has = base + lane < nq;
+                const int li = Wq[has ? base + lane : nq - 1];
+                const int y = y0 + (li >> 5), x = x0 + (li & 31);
+                const uint32_t site = (uint32_t)y * (uint32_t)L + (uint32_t)x;
+                en.site = site;
+                const SiteMean s = site_mean(A, A.in + A.it.off[k], L, y, x, cs.x);
+                double rs = 0.0;               // also where the neighbours cancel or their sum underflows
+                if (SAMP == 2) {
+                    rs = cs.z * s.cur + cs.w * s.alpha;
+                } else {
+                    const U4 r = philox4x32_10(site, (uint32_t)(unsigned long long)step, 0u,
+                                               (uint32_t)((unsigned long long)step >> 32), (uint32_t)seed,
+                                               (uint32_t)(seed >> 32));
+                    const uint32_t hm = hi32(s.m), hmu = hi32(s.mu1);
+                    const bool live = !(tmf::is_zero(s.alpha) && tmf::is_zero(s.cur));
+                    const bool draw = !tmf::is_zero(s.m);
+                    // above 100 by the high word: 100 itself has it too, and takes list 0
+                    const bool gauss = SAMP == 1 && live && hmu < 0x7ff00000u && hm >= 0x40590000u && hm < 0x7ff00000u;
+                    // m < 32 (not negative, not NaN), shape not negative, Inf or NaN
+                    const bool small = live && hmu < 0x7ff00000u && hm < 0x40400000u;
+                    if (live && !small) outcome = 0;
+                    const int n = search_count(small && draw, small ? tmf::trunc_f32(s.m) : 0.0f, r.x, tab.rcpf + 3);
+                    if (small && draw && n < 0) outcome = 0;
+                    if (SAMP == 1 && __any_sync(0xffffffffu, gauss)) {
+                        // Gaussian approximations of both draws: one ziggurat word each
+                        if (gauss && s.m > 100.0) {
+                            const int32_t h1 = zig_value(r.x), h2 = zig_value(r.y);
+                            const ZigLayer<double> l1 = tab.zig[zig_layer(r.x)], l2 = tab.zig[zig_layer(r.y)];
+                            const uint32_t a1 = (uint32_t)(h1 < 0 ? -h1 : h1), a2 = (uint32_t)(h2 < 0 ? -h2 : h2);
+                            const double kk = s.mu1 + trunc(tmf::mul(signed_mul(h1, l1.w), tmf::sqrt(s.m)) + s.m);
+                            if (a1 < l1.k && a2 < l2.k && kk > 100.0) {
+                                rs = (tmf::mul(signed_mul(h2, l2.w), tmf::sqrt(kk)) + kk) * cs.y;
+                                outcome = -1;
+                            }
+                        }
+                        __syncwarp();
+                    }
+                    const bool gamma = small && outcome < 0;
+                    if (__any_sync(0xffffffffu, gamma)) {
+                        const double kg = gamma ? s.mu1 + tmf::from_u31(draw ? (uint32_t)n : 0u) : 1.0;
+                        const uint32_t hk = hi32(kg);
+                        const uint32_t wz = draw ? r.y : r.x, wu = draw ? r.z : r.y;
+                        const bool boost = hk < 0x3ff00000u;
+                        const double d = (kg + (boost ? 1.0 : 0.0)) - 1.0 / 3.0;
+                        const double c = Tr<double>::inv_sqrt(9.0 * d);
+                        const int32_t hz = zig_value(wz);
+                        const uint32_t az = (uint32_t)(hz < 0 ? -hz : hz);
+                        const ZigLayer<double> lz = tab.zig[zig_layer(wz)];
+                        const double xz = signed_mul(hz, lz.w);
+                        const double v = 1.0 + c * xz;
+                        const float vf = tmf::trunc_f32(v), xf = tmf::trunc_f32(tmf::abs_bits(xz)), x2f = xf * xf;
+                        // squeeze with room for the FP32 roundings; 1 - u is at least ~wu 2^-32
+                        const float lhs = ((float)(~wu) * 0x1p-32f) * ((108.0f * tmf::trunc_f32(d)) * (vf < 1.0f ? vf : 1.0f));
+                        const bool ok = az < lz.k && (int32_t)hi32(v) > 0 && lhs > (x2f * x2f) * 1.0001f;
+                        const double res = tmf::mul_normal(d, tmf::mul_normal(tmf::mul_normal(v, v), v));
+                        if (gamma && !tmf::is_zero(kg)) {              // Gamma(0) = 0
+                            if (SAMP == 1 && hk >= 0x40590000u) {
+                                outcome = 0;
+                            } else if (!ok) {
+                                outcome = 1;
+                                en.b = draw ? 1.0 : 0.0;
+                            } else if (boost) {
+                                outcome = 2;
+                                en.b = tmf::with_sign(res, !draw);
+                            } else {
+                                rs = res * cs.y;
+                            }
+                            en.a = kg;
+                        }
+                        __syncwarp();
+                    }
+                }
+                if (!has) outcome = 3;
+                if (outcome < 0) store_site<REM>(A, k, site, rs, 0u);
+                __syncwarp();
+            }
+#pragma unroll
+            for (int l = 0; l < 3; ++l) {
+                const unsigned bal = __ballot_sync(0xffffffffu, outcome == l);
+                if (outcome == l) lists[l * kListCap + cnt[l] + __popc(bal & lt_mask)] = en;
+                cnt[l] += __popc(bal);
+            }
+            __syncwarp();
+            // full lists are drawn 32 entries at a time.  On the last trip what the block's
+            // warps still carry is joined, so that it takes as few passes as it can and
+            // the passes run on different warps.
+            if (!more) {
+                if (lane < 3) left[warp][lane] = lane == 0 ? cnt[0] : (lane == 1 ? cnt[1] : cnt[2]);
+                __syncthreads();
+            }
+            for (int job = warp;; job += kWarps) {
+                int l, at = 0;
+                const ListEntry* e = lists;
+                bool on = true;
+                if (more) {
+                    l = cnt[2] >= 32 ? 2 : (cnt[0] >= 32 ? 0 : 1);
+                    at = (l == 2 ? cnt[2] : (l == 0 ? cnt[0] : cnt[1])) - 32;
+                    if (at < 0) break;
+                    if (l == 2) cnt[2] = at;
+                    else if (l == 0) cnt[0] = at;
+                    else cnt[1] = at;
+                    e += l * kListCap + at + lane;
+                } else {
+                    // job -> list and 32 of the joined entries: the general draws first
+                    int j = job;
+                    for (l = 0; l < 3; ++l) {
+                        int n = 0;
+                        for (int w = 0; w < kWarps; ++w) n += left[w][l];
+                        const int passes = (n + 31) / 32;
+                        if (j < passes) break;
+                        j -= passes;
+                    }
+                    if (l == 3) break;
+                    int i = j * 32 + lane;
+                    on = false;
+                    for (int w = 0; w < kWarps; ++w) {
+                        const int n = left[w][l];
+                        if (!on && i < n) {
+                            on = true;
+                            e = reinterpret_cast<const ListEntry*>(smem_raw + w * warp_bytes(A.rows_cap)) + l * kListCap + i;
+                        }
+                        i -= n;
+                    }
+                }
+                if (l == 2) {
+                    if (on) draw_boost<REM>(A, step, *e);
+                } else {
+                    if (on) draw_general<REM, SAMP, CAP>(A, tab, step, l == 0, *e);
+                }
+                __syncwarp();
+            }
+            base += 32;
+        } while (base < nq);
+        if (!more) break;
+        __syncwarp();
+    }
+}
+
+namespace {
+
+template <int REM, int SAMP, int CAP = kSamplerCap>
+cudaError_t launch64_t(const DornicArgs<double>& a, int grid, int block, cudaStream_t s)
+{
+    static bool attr_set = false;
+    if (!attr_set) {
+        const cudaError_t e = cudaFuncSetAttribute(dornic_step64_kernel<REM, SAMP, CAP>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)(warp_bytes(kMaxRowsPerTask) * kWarps));
+        if (e != cudaSuccess) return e;
+        attr_set = true;
+    }
+    dornic_step64_kernel<REM, SAMP, CAP><<<grid, block, warp_bytes(a.rows_cap) * kWarps, s>>>(a);
+    return cudaGetLastError();
+}
+
+template <int REM>
+cudaError_t launch64_r(const DornicArgs<double>& a, int grid, int block, cudaStream_t s)
+{
+    if (a.cap1) {  // the sampler-cap probe: DP, Euler-exact remainder, exact sampler only
+        if (REM == 0 && a.sampler == 0) return launch64_t<0, 0, 1>(a, grid, block, s);
+        return cudaErrorInvalidValue;
+    }
+    if (a.sampler == 0) return launch64_t<REM, 0>(a, grid, block, s);
+    if (a.sampler == 1) return launch64_t<REM, 1>(a, grid, block, s);
+    if (a.sampler == 2) return launch64_t<REM, 2>(a, grid, block, s);
+    return cudaErrorInvalidValue;
+}
+
+}  // namespace
+
+template <>
+cudaError_t launch_dornic<double>(const DornicArgs<double>& a, int rem, int grid, int block, cudaStream_t s)
+{
+    if (a.n_tasks <= 0) return cudaSuccess;
+    if (block != 32 * kWarps || a.rows_cap < 1 || a.rows_cap > kMaxRowsPerTask) return cudaErrorInvalidValue;
+    if (rem == 0) return launch64_r<0>(a, grid, block, s);
+    if (rem == 1) return launch64_r<1>(a, grid, block, s);
+    if (rem == 2) return launch64_r<2>(a, grid, block, s);
+    return cudaErrorInvalidValue;
+}
+
+}  // namespace tmg
