@@ -143,6 +143,31 @@ int default_rows(const tm_batch* b)
     return R;
 }
 
+// Rows of the FP64 RK4 tiles: 24 or 12, whichever leaves the busiest SM fewer warps of
+// cells to evaluate over the four stages.  The shorter tile repeats more of its halo
+// (1.34 evaluations per cell and stage against 1.18) but spreads small batches over more
+// SMs and wastes less on ragged sides.
+int rk64_tile_rows(const tm_batch* b)
+{
+    int best = RK64_TY;
+    long long least = -1;
+    for (int ty = RK64_TY; ty >= RK64_UNIT; ty -= RK64_UNIT) {
+        long long tiles = 0, warps = 0;
+        for (int k = 0; k < b->n_inst; ++k) {
+            const long long L = b->inst[k].L;
+            tiles += ((L + ty - 1) / ty) * ((L + RK_TX - 1) / RK_TX);
+        }
+        for (int s = 0; s < 4; ++s) {
+            const int in = s + 1;
+            const long long ring = (long long)(RK_RX - 2 * in) * (ty + 2 * RK_H - 2 * in) - (long long)RK_TX * ty;
+            warps += RK_TX * ty / 32 + (ring + 31) / 32;
+        }
+        const long long sms = std::max(1, b->ctx->num_sms), cost = (tiles + sms - 1) / sms * warps;
+        if (least < 0 || cost < least) { least = cost; best = ty; }
+    }
+    return best;
+}
+
 int build_tasks(tm_batch* b)
 {
     // warp tasks
@@ -165,13 +190,14 @@ int build_tasks(tm_batch* b)
     TM_CUDA(cudaMemcpy(b->d_tasks, tasks.data(), tasks.size() * sizeof(int4), cudaMemcpyHostToDevice));
     if (!b->d_task_begin) TM_CUDA(dalloc(&b->d_task_begin, begin.size()));
     TM_CUDA(cudaMemcpy(b->d_task_begin, begin.data(), begin.size() * sizeof(int), cudaMemcpyHostToDevice));
-    // 64 x 32 tiles (Rietkerk RK4, noise-off DP)
+    // 64 x 32 tiles (Rietkerk RK4, noise-off DP; FP64 Rietkerk: rk64_tile_rows)
     if ((b->model == 1 || b->dpm.deterministic) && !b->d_btasks) {
         std::vector<int4> bt;
+        const int ty = (b->model == 1 && b->precision == TM_FP64) ? rk64_tile_rows(b) : RK_TY;
         for (int k = 0; k < b->n_inst; ++k) {
             const int L = b->inst[k].L;
-            for (int y0 = 0; y0 < L; y0 += RK_TY)
-                for (int x0 = 0; x0 < L; x0 += RK_TX) bt.push_back(make_int4(k, x0, y0, 0));
+            for (int y0 = 0; y0 < L; y0 += ty)
+                for (int x0 = 0; x0 < L; x0 += RK_TX) bt.push_back(make_int4(k, x0, y0, ty));
         }
         b->n_btasks = (int)bt.size();
         TM_CUDA(dalloc(&b->d_btasks, bt.size()));
@@ -295,7 +321,7 @@ cudaError_t enqueue_step_t(tm_batch* b, int src_idx, const long long* step_base,
         return e;
     }
     const tm_rietkerk_model& m = b->rkm;
-    const int grid_rk = std::max(1, std::min(b->n_btasks, b->ctx->num_sms * RK_CTAS));
+    const int grid_rk = std::max(1, std::min(b->n_btasks, b->ctx->num_sms * (sizeof(T) == 8 ? 1 : RK_CTAS)));
     if (m.deterministic) {
         RK4Args<T> r = rk4_args<T>(b, in, nullptr, out);
         return launch_rk4<T>(r, true, grid_rk, s);

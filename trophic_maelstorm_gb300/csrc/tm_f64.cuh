@@ -166,13 +166,17 @@ TM_HD double mul_normal(double a, double b)
     return bits_f64(r | ((ua ^ ub) & kSign));
 }
 
-// a b for any operands
+// a b for any operands (a zero with a finite operand, common on empty lattices, stays
+// on the integer pipe)
 TM_HD double mul(double a, double b)
 {
     const uint64_t ua = f64_bits(a), ub = f64_bits(b);
     const int ea = f64_exp_field(ua), eb = f64_exp_field(ub);
     int e = ea + eb - 1023;
-    if (!(field_normal(ea) && field_normal(eb) && (uint32_t)(e - 2) < 2042u)) return hw_mul(a, b);
+    if (!(field_normal(ea) && field_normal(eb) && (uint32_t)(e - 2) < 2042u)) {
+        if (((ua << 1) == 0 || (ub << 1) == 0) && ea < 2047 && eb < 2047) return bits_f64((ua ^ ub) & kSign);
+        return hw_mul(a, b);
+    }
     const uint64_t r = mul_core(ua, ub, e);
     return bits_f64(r | ((ua ^ ub) & kSign));
 }
@@ -219,16 +223,23 @@ TM_HD bool div_fields_ok(int ea, int eb)
     return field_normal(ea) && field_normal(eb) && (uint32_t)(ea - eb + 1023 - 2) < 2043u;
 }
 
-// a / b for any operands
-TM_HD double div(double a, double b)
+// a / b with b's reciprocal R where b is normal
+TM_HD double div_by(double a, double b, uint32_t R)
 {
     const uint64_t ua = f64_bits(a), ub = f64_bits(b);
     const int ea = f64_exp_field(ua), eb = f64_exp_field(ub);
-    if (!div_fields_ok(ea, eb)) return hw_div(a, b);
+    if (!div_fields_ok(ea, eb)) {
+        if ((ua << 1) == 0 && field_normal(eb)) return bits_f64((ua ^ ub) & kSign);
+        return hw_div(a, b);
+    }
     int e = ea - eb + 1023;
-    const uint64_t r = div_core(ua, ub, recip31((ub & kFrac) | kOne), e);
+    const uint64_t r = div_core(ua, ub, R, e);
     return bits_f64(r | ((ua ^ ub) & kSign));
 }
+TM_HD uint32_t recip_of(double b) { return recip31((f64_bits(b) & kFrac) | kOne); }
+
+// a / b for any operands
+TM_HD double div(double a, double b) { return div_by(a, b, recip_of(b)); }
 
 // ---------------------------------------------------------------- square root
 // sqrt of a positive normal number: a 32-bit root from the FP32 estimate and one

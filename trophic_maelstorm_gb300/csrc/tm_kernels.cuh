@@ -30,7 +30,7 @@ struct InstTables {
 };
 
 // Warp task: 32 columns x `rows` rows of one instance: (inst, x0, y0, rows).
-// Block task (RK4 tile): (inst, x0, y0, 0).
+// Block task (RK4 tile): (inst, x0, y0, tile rows).
 
 template <typename T>
 struct DornicArgs {
@@ -89,6 +89,10 @@ template <>   // tm_step64.cu
 cudaError_t launch_dornic<double>(const DornicArgs<double>& a, int rem, int grid, int block, cudaStream_t s);
 template <typename T>
 cudaError_t launch_rk4(const RK4Args<T>& a, bool det, int grid, cudaStream_t s);
+template <>
+cudaError_t launch_rk4<float>(const RK4Args<float>& a, bool det, int grid, cudaStream_t s);
+template <>
+cudaError_t launch_rk4<double>(const RK4Args<double>& a, bool det, int grid, cudaStream_t s);
 template <typename T>
 cudaError_t launch_measure(const T* state, const InstTables& it, const int4* tasks, int n_tasks, int nf,
                            double* partial, int grid, int block, cudaStream_t s, int spread = 0, int cx = -1,
@@ -113,6 +117,8 @@ constexpr int kMaxRowsPerTask = 16;
 constexpr int RK_TX = 64, RK_TY = 32, RK_H = 4;
 constexpr int RK_RX = RK_TX + 2 * RK_H, RK_RY = RK_TY + 2 * RK_H, RK_RN = RK_RX * RK_RY;
 constexpr int RK_THREADS = 512;
+constexpr int RK64_THREADS = 768;          // FP64 RK4 tiles: threads, and rows of the tallest tile
+constexpr int RK64_UNIT = RK64_THREADS / RK_TX, RK64_TY = 32 / RK64_UNIT * RK64_UNIT;
 constexpr int RK_CTAS = 2;                 // resident RK4 tile CTAs per SM (FP32)
 
 }  // namespace tmg

@@ -25,33 +25,26 @@ __device__ __forceinline__ T add_pow2_times(T c, T s, T x)
 }
 
 // Right-hand side at region cell c of S (f_2Dor, or f_2D when DET); R per instance.
-template <typename T, bool DET>
-__device__ __forceinline__ void rk_rhs_cell(const RK4Args<T>& A, const T* S, int c, T R, T& fP, T& fW, T& fO)
+template <bool DET>
+__device__ __forceinline__ void rk_rhs_cell(const RK4Args<float>& A, const float* S, int c, float R, float& fP, float& fW,
+                                            float& fO)
 {
     const int cn = c - RK_RX, cs = c + RK_RX, cw = c - 1, ce = c + 1;
-    const T* SP = S;
-    const T* SW = S + RK_RN;
-    const T* SO = S + 2 * RK_RN;
-    const T Pc = SP[c], Wc = SW[c], Oc = SO[c];
-    const T upt_num = (A.gmax * Wc) * Pc;
-    const T wk = Wc + A.k1;
-    T infil, upt;
-    if constexpr (sizeof(T) == 8) {
-        // the reference's own expressions
-        infil = ((A.alpha * (Pc + A.k2W0)) / (Pc + A.k2)) * Oc;
-        fP = ((A.cgmax * Wc) * Pc) / wk;
-        upt = upt_num / wk;
-    } else {
-        // FP32: two correctly rounded reciprocals instead of three divisions
-        const T iwk = __frcp_rn(wk);
-        infil = ((A.alpha * (Pc + A.k2W0)) * __frcp_rn(Pc + A.k2)) * Oc;
-        fP = ((A.cgmax * Wc) * Pc) * iwk;
-        upt = upt_num * iwk;
-    }
-    const T lapW = add_pow2_times(((SW[cn] + SW[cs]) + SW[cw]) + SW[ce], T(-4), Wc);
-    const T lapO = add_pow2_times(((SO[cn] + SO[cs]) + SO[cw]) + SO[ce], T(-4), Oc);
+    const float* SP = S;
+    const float* SW = S + RK_RN;
+    const float* SO = S + 2 * RK_RN;
+    const float Pc = SP[c], Wc = SW[c], Oc = SO[c];
+    const float upt_num = (A.gmax * Wc) * Pc;
+    const float wk = Wc + A.k1;
+    // two correctly rounded reciprocals instead of three divisions
+    const float iwk = __frcp_rn(wk);
+    const float infil = ((A.alpha * (Pc + A.k2W0)) * __frcp_rn(Pc + A.k2)) * Oc;
+    fP = ((A.cgmax * Wc) * Pc) * iwk;
+    const float upt = upt_num * iwk;
+    const float lapW = add_pow2_times(((SW[cn] + SW[cs]) + SW[cw]) + SW[ce], -4.0f, Wc);
+    const float lapO = add_pow2_times(((SO[cn] + SO[cs]) + SO[cw]) + SO[ce], -4.0f, Oc);
     if (DET) {
-        const T lapP = add_pow2_times(((SP[cn] + SP[cs]) + SP[cw]) + SP[ce], T(-4), Pc);
+        const float lapP = add_pow2_times(((SP[cn] + SP[cs]) + SP[cw]) + SP[ce], -4.0f, Pc);
         fP = (fP - A.d * Pc) + A.DPx * lapP;
     }
     fW = ((infil - upt) - A.rW * Wc) + A.DWx * lapW;
@@ -63,11 +56,11 @@ __device__ __forceinline__ void rk_rhs_cell(const RK4Args<T>& A, const T* S, int
 // interior cell depends on -- so the interior is exact after stage 3.  Stage
 // inputs ping-pong between two shared buffers, so each stage needs one barrier
 // and no value is held in registers across it.
-// Tile rows by bulk copy: for a tile that does not wrap in x on a lattice with
-// L % 4 == 0, each of the 3 x RK_RY halo rows is a contiguous RK_RX-float segment
-// starting on a 16-byte boundary (instance offsets and field strides are
-// multiples of 32 elements), so one thread issues them as cp.async.bulk copies
-// completing on an mbarrier instead of 256 threads loading 5184 values.
+// Tile rows by bulk copy: for a tile that does not wrap in x on a lattice whose rows
+// are multiples of 16 bytes, each of the halo rows is a contiguous segment of RK_RX
+// values starting on a 16-byte boundary (instance offsets and field strides are
+// multiples of 32 elements), so one thread per row and field issues it as a cp.async.bulk copy
+// completing on an mbarrier instead of every thread loading values.
 // Every wait on the copies is bounded (RK4Args::wait_limit polls, about 0.3 s at
 // the default): a CTA whose copies do not complete marks the instances of its
 // current and remaining tiles with TM_STATUS_WAIT_BIT (their fields are invalid
@@ -91,15 +84,87 @@ __device__ __forceinline__ bool rk_bar_wait(uint32_t bar, uint32_t parity, int l
     return false;
 }
 
-template <typename T, bool DET>
-__global__ void __launch_bounds__(RK_THREADS, (sizeof(T) == 4 ? RK_CTAS : 1)) rk4_tile_kernel(const RK4Args<T> A)
+// The region of tile t (RK_RX columns x ry_n rows of P, W, O, periodic) into X0.  False
+// when its copies did not complete: the instances are flagged and the block returns.
+template <typename T>
+__device__ __forceinline__ bool load_tile(const RK4Args<T>& A, T* X0, int ry_n, const T* __restrict__ P0,
+                                          const T* __restrict__ W0, const T* __restrict__ O0, int L, int x0, int y0, int t,
+                                          uint32_t bar, uint32_t& phase)
+{
+    const int tid = threadIdx.x, rn = RK_RX * ry_n;
+    __syncthreads();  // previous tile done with shared memory
+    // halo coordinates lie within RK_H of [0, L + tile), so one wrap is enough
+    // once L covers the tile and its halo; smaller lattices take the modulo
+    const bool one_wrap = L >= ry_n && L >= RK_RX;
+    // one halo row per thread (3 x ry_n rows): the block takes the bulk path only if
+    // every row start is 16-byte aligned
+    const int n_rows = 3 * ry_n;
+    const bool shape = (one_wrap && (L * sizeof(T)) % 16 == 0 && x0 >= RK_H && x0 + RK_TX + RK_H <= L) || A.probe_no_copy;
+    const T* src = nullptr;
+    bool aligned = true;
+    if (shape && !A.probe_no_copy && tid < n_rows) {
+        const int f = tid / ry_n, ry = tid - f * ry_n;
+        int gy = y0 - RK_H + ry;
+        gy = gy < 0 ? gy + L : (gy >= L ? gy - L : gy);
+        src = (f == 0 ? P0 : (f == 1 ? W0 : O0)) + (long long)gy * L + (x0 - RK_H);
+        aligned = ((uintptr_t)src & 15u) == 0;
+    }
+    if (shape && __syncthreads_and(aligned)) {
+        if (!A.probe_no_copy) {
+            constexpr uint32_t row_bytes = RK_RX * sizeof(T);
+            static_assert((RK_RX * sizeof(float)) % 16 == 0, "bulk rows");
+            if (tid == 0)
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+                             :: "r"(bar), "r"((uint32_t)n_rows * row_bytes) : "memory");
+            __syncthreads();
+            if (tid < n_rows) {
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes "
+                             "[%0], [%1], %2, [%3];"
+                             :: "r"(rk_saddr(X0 + tid * RK_RX)), "l"(src), "r"(row_bytes), "r"(bar)
+                             : "memory");
+            }
+        }
+        const bool ok = rk_bar_wait(bar, phase, A.wait_limit);
+        phase ^= 1u;
+        if (__syncthreads_or(!ok)) {
+            // copies did not complete: flag this tile's and every later tile's
+            // instance, give copies still in flight one more bounded wait, stop
+            for (int t2 = t + tid * (int)gridDim.x; t2 < A.n_tasks; t2 += (int)blockDim.x * (int)gridDim.x)
+                atomicOr(A.it.status + A.tasks[t2].x, TM_STATUS_WAIT_BIT);
+            (void)rk_bar_wait(bar, phase ^ 1u, A.wait_limit);
+            return false;
+        }
+    } else {
+#pragma unroll 2
+        for (int c = tid; c < rn; c += (int)blockDim.x) {
+            const int ry = c / RK_RX, rx = c - ry * RK_RX;
+            int gy = y0 - RK_H + ry, gx = x0 - RK_H + rx;
+            if (one_wrap) {
+                gy = gy < 0 ? gy + L : (gy >= L ? gy - L : gy);
+                gx = gx < 0 ? gx + L : (gx >= L ? gx - L : gx);
+            } else {
+                gy %= L; if (gy < 0) gy += L;
+                gx %= L; if (gx < 0) gx += L;
+            }
+            const long long gi = (long long)gy * L + gx;
+            X0[c] = P0[gi];
+            X0[rn + c] = W0[gi];
+            X0[2 * rn + c] = O0[gi];
+        }
+        __syncthreads();
+    }
+    return true;
+}
+
+template <bool DET>
+__global__ void __launch_bounds__(RK_THREADS, RK_CTAS) rk4_tile_kernel(const RK4Args<float> A)
 {
     extern __shared__ __align__(16) unsigned char rk_smem[];
     __shared__ __align__(8) uint64_t tile_bar;
-    __shared__ int tile_bulk;
-    T* const X0 = reinterpret_cast<T*>(rk_smem);          // [3][RK_RN] stage-0 input
-    T* const MA = X0 + 3 * RK_RN;                           // [3][RK_RN] stage inputs (ping)
-    T* const MB = MA + 3 * RK_RN;                           // [3][RK_RN] (pong)
+    float* const X0 = reinterpret_cast<float*>(rk_smem);          // [3][RK_RN] stage-0 input
+    float* const MA = X0 + 3 * RK_RN;                           // [3][RK_RN] stage inputs (ping)
+    float* const MB = MA + 3 * RK_RN;                           // [3][RK_RN] (pong)
     constexpr int kPer = RK_TX * RK_TY / RK_THREADS;        // interior cells per thread
     static_assert(RK_TX * RK_TY % RK_THREADS == 0, "interior cells per thread");
     const int tid = threadIdx.x;
@@ -116,101 +181,35 @@ __global__ void __launch_bounds__(RK_THREADS, (sizeof(T) == 4 ? RK_CTAS : 1)) rk
         const int L = A.it.L[k];
         const long long off = A.it.off[k];
         const long long fs = A.it.fstride[k];
-        const T R = (T)A.it.R[k];
+        const float R = (float)A.it.R[k];
         const int x0 = tk.y, y0 = tk.z;
-        const T* __restrict__ P0 = (DET ? A.in : A.pstar) + off;
-        const T* __restrict__ W0 = A.in + off + fs;
-        const T* __restrict__ O0 = A.in + off + 2 * fs;
-        __syncthreads();  // previous tile done with shared memory
-        // halo coordinates lie within RK_H of [0, L + tile), so one wrap is enough
-        // once L covers the tile and its halo; smaller lattices take the modulo
-        const bool one_wrap = L >= RK_RY && L >= RK_RX;
-        {
-            // one halo row per thread (3 x RK_RY rows): the block takes the bulk path
-            // only if every row start is 16-byte aligned
-            constexpr int kRows = 3 * RK_RY;
-            const bool shape = (sizeof(T) == 4 && one_wrap && (L & 3) == 0 && x0 >= RK_H && x0 + RK_TX + RK_H <= L) ||
-                               A.probe_no_copy;
-            const T* src = nullptr;
-            bool aligned = true;
-            if (shape && !A.probe_no_copy && tid < kRows) {
-                const int f = tid / RK_RY, ry = tid - f * RK_RY;
-                int gy = y0 - RK_H + ry;
-                gy = gy < 0 ? gy + L : (gy >= L ? gy - L : gy);
-                src = (f == 0 ? P0 : (f == 1 ? W0 : O0)) + (long long)gy * L + (x0 - RK_H);
-                aligned = ((uintptr_t)src & 15u) == 0;
-            }
-            const bool bulk = shape && __syncthreads_and(aligned);
-            if (bulk && !A.probe_no_copy) {
-                constexpr uint32_t row_bytes = RK_RX * sizeof(T);
-                static_assert((RK_RX * sizeof(float)) % 16 == 0 && (RK_RN * sizeof(float)) % 16 == 0, "bulk rows");
-                if (tid == 0)
-                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
-                                 :: "r"(bar), "r"((uint32_t)kRows * row_bytes) : "memory");
-                __syncthreads();
-                if (tid < kRows) {
-                    const int f = tid / RK_RY, ry = tid - f * RK_RY;
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes "
-                                 "[%0], [%1], %2, [%3];"
-                                 :: "r"(rk_saddr(X0 + f * RK_RN + ry * RK_RX)), "l"(src), "r"(row_bytes), "r"(bar)
-                                 : "memory");
-                }
-            }
-            if (tid == 0) tile_bulk = bulk ? 1 : 0;
-        }
-        __syncthreads();
-        if (tile_bulk) {
-            const bool ok = rk_bar_wait(bar, phase, A.wait_limit);
-            phase ^= 1u;
-            if (__syncthreads_or(!ok)) {
-                // copies did not complete: flag this tile's and every later tile's
-                // instance, give copies still in flight one more bounded wait, stop
-                for (int t2 = t + tid * (int)gridDim.x; t2 < A.n_tasks; t2 += RK_THREADS * (int)gridDim.x)
-                    atomicOr(A.it.status + A.tasks[t2].x, TM_STATUS_WAIT_BIT);
-                (void)rk_bar_wait(bar, phase ^ 1u, A.wait_limit);
-                return;
-            }
-        } else
-        for (int c = tid; c < RK_RN; c += RK_THREADS) {
-            const int ry = c / RK_RX, rx = c - ry * RK_RX;
-            int gy = y0 - RK_H + ry, gx = x0 - RK_H + rx;
-            if (one_wrap) {
-                gy = gy < 0 ? gy + L : (gy >= L ? gy - L : gy);
-                gx = gx < 0 ? gx + L : (gx >= L ? gx - L : gx);
-            } else {
-                gy %= L; if (gy < 0) gy += L;
-                gx %= L; if (gx < 0) gx += L;
-            }
-            const long long gi = (long long)gy * L + gx;
-            X0[c] = P0[gi];
-            X0[RK_RN + c] = W0[gi];
-            X0[2 * RK_RN + c] = O0[gi];
-        }
-        __syncthreads();
+        const float* __restrict__ P0 = (DET ? A.in : A.pstar) + off;
+        const float* __restrict__ W0 = A.in + off + fs;
+        const float* __restrict__ O0 = A.in + off + 2 * fs;
+        if (!load_tile<float>(A, X0, RK_RY, P0, W0, O0, L, x0, y0, t, bar, phase)) return;
         // Stage s on the region inset by s+1: the 64 x 32 interior with a fixed
         // thread mapping (kPer cells per thread, whose weighted sums of K stay in
         // registers), then the ring between the inset and the interior.
-        T acc[3][kPer];
+        float acc[3][kPer];
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
-            const T* S = (s == 0) ? X0 : ((s & 1) ? MA : MB);
-            T* D = (s & 1) ? MB : MA;
-            const T coef = (s == 2) ? A.dt : A.dt2;
+            const float* S = (s == 0) ? X0 : ((s & 1) ? MA : MB);
+            float* D = (s & 1) ? MB : MA;
+            const float coef = (s == 2) ? A.dt : A.dt2;
 #pragma unroll
             for (int j = 0; j < kPer; ++j) {
                 const int a = tid + j * RK_THREADS;
                 const int c = ((a / RK_TX) + RK_H) * RK_RX + (a % RK_TX) + RK_H;
-                T k0, k1, k2;
-                rk_rhs_cell<T, DET>(A, S, c, R, k0, k1, k2);
+                float k0, k1, k2;
+                rk_rhs_cell<DET>(A, S, c, R, k0, k1, k2);
                 if (s == 0) {
                     acc[0][j] = k0; acc[1][j] = k1; acc[2][j] = k2;
                 } else if (s == 3) {
                     acc[0][j] = acc[0][j] + k0; acc[1][j] = acc[1][j] + k1; acc[2][j] = acc[2][j] + k2;
                 } else {
-                    acc[0][j] = add_pow2_times(acc[0][j], T(2), k0);
-                    acc[1][j] = add_pow2_times(acc[1][j], T(2), k1);
-                    acc[2][j] = add_pow2_times(acc[2][j], T(2), k2);
+                    acc[0][j] = add_pow2_times(acc[0][j], 2.0f, k0);
+                    acc[1][j] = add_pow2_times(acc[1][j], 2.0f, k1);
+                    acc[2][j] = add_pow2_times(acc[2][j], 2.0f, k2);
                 }
                 if (s < 3) {
                     D[c] = X0[c] + coef * k0;
@@ -236,8 +235,8 @@ __global__ void __launch_bounds__(RK_THREADS, (sizeof(T) == 4 ? RK_CTAS : 1)) rk
                         rx = (qs < nside ? in : RK_H + RK_TX) + qq % t;
                     }
                     const int c = ry * RK_RX + rx;
-                    T k0, k1, k2;
-                    rk_rhs_cell<T, DET>(A, S, c, R, k0, k1, k2);
+                    float k0, k1, k2;
+                    rk_rhs_cell<DET>(A, S, c, R, k0, k1, k2);
                     D[c] = X0[c] + coef * k0;
                     D[RK_RN + c] = X0[RK_RN + c] + coef * k1;
                     D[2 * RK_RN + c] = X0[2 * RK_RN + c] + coef * k2;
@@ -256,8 +255,8 @@ __global__ void __launch_bounds__(RK_THREADS, (sizeof(T) == 4 ? RK_CTAS : 1)) rk
                 const long long gi = off + (long long)gy * L + gx;
 #pragma unroll
                 for (int f = 0; f < 3; ++f) {
-                    T v = X0[f * RK_RN + c] + A.dt6 * acc[f][j];
-                    if (v < A.ceps && v >= A.clo) v = T(0);
+                    float v = X0[f * RK_RN + c] + A.dt6 * acc[f][j];
+                    if (v < A.ceps && v >= A.clo) v = 0.0f;
                     st |= value_status(v);
                     A.out[gi + f * fs] = v;
                 }
@@ -267,25 +266,204 @@ __global__ void __launch_bounds__(RK_THREADS, (sizeof(T) == 4 ? RK_CTAS : 1)) rk
     }
 }
 
-template <typename T>
-cudaError_t launch_rk4(const RK4Args<T>& a, bool det, int grid, cudaStream_t s)
+// ---- the same step in FP64
+// The FP64 pipe takes one warp instruction per 64-76 cycles, so the products run on the
+// integer pipe and the quotients are exact integer divisions, the two by W + k1 sharing
+// its reciprocal (tm_f64.cuh): 22 FP64 instructions per cell and stage, all of them
+// additions, where the plain expressions took 58.  An evaluation is then some 900
+// instructions long, so the code has one copy of it: one loop over the interior and
+// ring cells of a stage, the stage a loop variable, and the weighted stage sums of a
+// thread's interior cells rotating through fixed registers.  Tiles are 64 columns x
+// tk.w rows (rk64_tile_rows, tm_capi.cu).
+// Bound by the FP64 and the integer pipe taking turns (61 % and 46 % busy, 41 % of the
+// issue slots): 768 threads (6 warps per scheduler, 76 registers) took 9.3 ms for 20 steps
+// of 16 lattices of 256^2, 512 threads 10.1 and 1024 9.7; with some products back on the
+// FP64 pipe 9.6 to 10.0.  The plain expressions took 15.2 ms (both with the draw of P*).
+__device__ __forceinline__ double clamp_zero(double v, double clo, double ceps)
+{
+    // not below ceps if positive with larger bits (a NaN neither)
+    const long long vb = __double_as_longlong(v);
+    if (!(vb >= 0 && vb >= __double_as_longlong(ceps)) && vb != 0) {
+        if (tmf::hw_in_range(v, clo, ceps)) return 0.0;
+    }
+    return v;
+}
+
+template <bool DET>
+__device__ __forceinline__ void rk_rhs_cell64(const RK4Args<double>& A, const double* S, int rn, int c, double R, double& fP,
+                                              double& fW, double& fO)
+{
+    const int cn = c - RK_RX, cs = c + RK_RX, cw = c - 1, ce = c + 1;
+    const double* SP = S;
+    const double* SW = S + rn;
+    const double* SO = S + 2 * rn;
+    const double Pc = SP[c], Wc = SW[c], Oc = SO[c];
+    const double wk = Wc + A.k1;
+    const uint32_t rw = tmf::recip_of(wk);
+    fP = tmf::div_by(tmf::mul(tmf::mul(A.cgmax, Wc), Pc), wk, rw);
+    const double upt = tmf::div_by(tmf::mul(tmf::mul(A.gmax, Wc), Pc), wk, rw);
+    const double infil = tmf::mul(tmf::div(tmf::mul(A.alpha, Pc + A.k2W0), Pc + A.k2), Oc);
+    const double lapW = add_pow2_times(((SW[cn] + SW[cs]) + SW[cw]) + SW[ce], -4.0, Wc);
+    const double lapO = add_pow2_times(((SO[cn] + SO[cs]) + SO[cw]) + SO[ce], -4.0, Oc);
+    if (DET) {
+        const double lapP = add_pow2_times(((SP[cn] + SP[cs]) + SP[cw]) + SP[ce], -4.0, Pc);
+        fP = (fP - tmf::mul(A.d, Pc)) + tmf::mul(A.DPx, lapP);
+    }
+    fW = ((infil - upt) - tmf::mul(A.rW, Wc)) + tmf::mul(A.DWx, lapW);
+    fO = (R - infil) + tmf::mul(A.DOx, lapO);
+}
+
+template <bool DET>
+__global__ void __launch_bounds__(RK64_THREADS, 1) rk4_tile64_kernel(const RK4Args<double> A)
+{
+    extern __shared__ __align__(16) unsigned char rk_smem[];
+    constexpr int kMax = RK_TX * RK64_TY / RK64_THREADS;        // interior cells per thread in the tallest tile
+    __shared__ __align__(8) uint64_t tile_bar;
+    const int tid = threadIdx.x;
+    const uint32_t bar = rk_saddr(&tile_bar);
+    if (tid == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(bar) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    uint32_t phase = 0;
+    for (int t = blockIdx.x; t < A.n_tasks; t += gridDim.x) {
+        const int4 tk = A.tasks[t];
+        const int k = tk.x;
+        const int L = A.it.L[k];
+        const long long off = A.it.off[k];
+        const long long fs = A.it.fstride[k];
+        const double R = A.it.R[k];
+        const int x0 = tk.y, y0 = tk.z, ty = tk.w;
+        const int ry_n = ty + 2 * RK_H, rn = RK_RX * ry_n;
+        const int per = RK_TX * ty / RK64_THREADS;
+        double* const X0 = reinterpret_cast<double*>(rk_smem);   // [3][rn] stage-0 input
+        double* const MA = X0 + 3 * rn;                            // [3][rn] stage inputs (ping)
+        double* const MB = MA + 3 * rn;                            // [3][rn] (pong)
+        const double* __restrict__ P0 = (DET ? A.in : A.pstar) + off;
+        const double* __restrict__ W0 = A.in + off + fs;
+        const double* __restrict__ O0 = A.in + off + 2 * fs;
+        if (!load_tile<double>(A, X0, ry_n, P0, W0, O0, L, x0, y0, t, bar, phase)) return;
+        double acc[3][kMax];
+#pragma unroll
+        for (int j = 0; j < kMax; ++j) acc[0][j] = acc[1][j] = acc[2][j] = 0.0;
+#pragma unroll 1
+        for (int s = 0; s < 4; ++s) {
+            const double* S = (s == 0) ? X0 : ((s & 1) ? MA : MB);
+            double* D = (s & 1) ? MB : MA;
+            const double coef = (s == 2) ? A.dt : A.dt2;
+            const double weight = (s == 0 || s == 3) ? 1.0 : 2.0;
+            // the interior (per cells of this thread), then the ring between the region
+            // inset by s + 1 and the interior: top and bottom bands (th rows of the
+            // inset's width w), left and right bands (ty rows, th columns)
+            const int in = s + 1, th = 3 - s, w = RK_RX - 2 * in;
+            const int nband = th * w, nside = ty * th, nring = 2 * nband + 2 * nside;
+#pragma unroll 1
+            for (int q = 0; q < per || tid + (q - per) * RK64_THREADS < nring; ++q) {
+                int rx, ry;
+                const bool inner = q < per;
+                if (inner) {
+                    const int a = tid + q * RK64_THREADS;
+                    ry = a / RK_TX + RK_H;
+                    rx = a % RK_TX + RK_H;
+                } else {
+                    const int a = tid + (q - per) * RK64_THREADS;
+                    if (a < 2 * nband) {
+                        const int b = a < nband ? a : a - nband;
+                        ry = (a < nband ? in : RK_H + ty) + b / w;
+                        rx = in + b % w;
+                    } else {
+                        const int b = a - 2 * nband, b2 = b < nside ? b : b - nside;
+                        ry = RK_H + b2 / th;
+                        rx = (b < nside ? in : RK_H + RK_TX) + b2 % th;
+                    }
+                }
+                const int c = ry * RK_RX + rx;
+                double k0, k1, k2;
+                rk_rhs_cell64<DET>(A, S, rn, c, R, k0, k1, k2);
+                if (inner) {
+                    // sums of K (weights 1, 2, 2, 1: each fused add rounds once, as k + 2 k'
+                    // does); the front moves to the back
+                    const double n0 = fma(weight, k0, acc[0][0]), n1 = fma(weight, k1, acc[1][0]),
+                                 n2 = fma(weight, k2, acc[2][0]);
+#pragma unroll
+                    for (int j = 0; j + 1 < kMax; ++j) {
+                        acc[0][j] = acc[0][j + 1]; acc[1][j] = acc[1][j + 1]; acc[2][j] = acc[2][j + 1];
+                    }
+                    acc[0][kMax - 1] = n0; acc[1][kMax - 1] = n1; acc[2][kMax - 1] = n2;
+                }
+                if (s < 3) {
+                    D[c] = X0[c] + tmf::mul(coef, k0);
+                    D[rn + c] = X0[rn + c] + tmf::mul(coef, k1);
+                    D[2 * rn + c] = X0[2 * rn + c] + tmf::mul(coef, k2);
+                }
+            }
+            for (int q = per; q < kMax; ++q) {               // shorter tiles: bring the first cell to the front
+                const double n0 = acc[0][0], n1 = acc[1][0], n2 = acc[2][0];
+#pragma unroll
+                for (int j = 0; j + 1 < kMax; ++j) {
+                    acc[0][j] = acc[0][j + 1]; acc[1][j] = acc[1][j + 1]; acc[2][j] = acc[2][j + 1];
+                }
+                acc[0][kMax - 1] = n0; acc[1][kMax - 1] = n1; acc[2][kMax - 1] = n2;
+            }
+            __syncthreads();
+        }
+        unsigned st = 0;
+#pragma unroll
+        for (int j = 0; j < kMax; ++j) {
+            const int a = tid + j * RK64_THREADS;
+            const int ly = a / RK_TX, lx = a % RK_TX;
+            const int gy = y0 + ly, gx = x0 + lx;
+            if (j < per && gy < L && gx < L) {
+                const int c = (ly + RK_H) * RK_RX + lx + RK_H;
+                const long long gi = off + (long long)gy * L + gx;
+#pragma unroll
+                for (int f = 0; f < 3; ++f) {
+                    const double v = clamp_zero(X0[f * rn + c] + A.dt6 * acc[f][j], A.clo, A.ceps);
+                    st |= value_status(v);
+                    A.out[gi + f * fs] = v;
+                }
+            }
+        }
+        if (st) atomicOr(A.it.status + k, st);
+    }
+}
+
+template <>
+cudaError_t launch_rk4<float>(const RK4Args<float>& a, bool det, int grid, cudaStream_t s)
 {
     if (a.n_tasks <= 0) return cudaSuccess;
-    const size_t smem = 9 * (size_t)RK_RN * sizeof(T);
+    const size_t smem = 9 * (size_t)RK_RN * sizeof(float);
     static bool attr[2] = {false, false};
-    cudaError_t e = cudaSuccess;
     if (!attr[det ? 1 : 0]) {
-        e = det ? cudaFuncSetAttribute(rk4_tile_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                : cudaFuncSetAttribute(rk4_tile_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t e =
+            det ? cudaFuncSetAttribute(rk4_tile_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+                : cudaFuncSetAttribute(rk4_tile_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         attr[det ? 1 : 0] = true;
     }
-    if (det) rk4_tile_kernel<T, true><<<grid, RK_THREADS, smem, s>>>(a);
-    else rk4_tile_kernel<T, false><<<grid, RK_THREADS, smem, s>>>(a);
+    if (det) rk4_tile_kernel<true><<<grid, RK_THREADS, smem, s>>>(a);
+    else rk4_tile_kernel<false><<<grid, RK_THREADS, smem, s>>>(a);
     return cudaGetLastError();
 }
-template cudaError_t launch_rk4<float>(const RK4Args<float>&, bool, int, cudaStream_t);
-template cudaError_t launch_rk4<double>(const RK4Args<double>&, bool, int, cudaStream_t);
+
+template <>
+cudaError_t launch_rk4<double>(const RK4Args<double>& a, bool det, int grid, cudaStream_t s)
+{
+    if (a.n_tasks <= 0) return cudaSuccess;
+    const size_t smem = 9 * (size_t)RK_RX * (RK64_TY + 2 * RK_H) * sizeof(double);   // of the tallest tile
+    static bool attr[2] = {false, false};
+    if (!attr[det ? 1 : 0]) {
+        const cudaError_t e =
+            det ? cudaFuncSetAttribute(rk4_tile64_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+                : cudaFuncSetAttribute(rk4_tile64_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        attr[det ? 1 : 0] = true;
+    }
+    if (det) rk4_tile64_kernel<true><<<grid, RK64_THREADS, smem, s>>>(a);
+    else rk4_tile64_kernel<false><<<grid, RK64_THREADS, smem, s>>>(a);
+    return cudaGetLastError();
+}
 
 // ---- noise-off DP: drho/dt = a rho - b rho^2 - c rho^3 + D Lap(rho) ---------------
 // percNoDiff_2D (stochasticSPDP.cpp:549-662) with the 5-point Laplacian or the
