@@ -119,6 +119,6 @@ constexpr int RK_RX = RK_TX + 2 * RK_H, RK_RY = RK_TY + 2 * RK_H, RK_RN = RK_RX 
 constexpr int RK_THREADS = 512;
 constexpr int RK64_THREADS = 768;          // FP64 RK4 tiles: threads, and rows of the tallest tile
 constexpr int RK64_UNIT = RK64_THREADS / RK_TX, RK64_TY = 32 / RK64_UNIT * RK64_UNIT;
-constexpr int RK_CTAS = 2;                 // resident RK4 tile CTAs per SM (FP32)
+constexpr int RK_CTAS = 2;                 // resident FP32 RK4 tile CTAs per SM
 
 }  // namespace tmg

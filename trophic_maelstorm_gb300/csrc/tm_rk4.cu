@@ -24,33 +24,6 @@ __device__ __forceinline__ T add_pow2_times(T c, T s, T x)
     return Tr<T>::fma_(s, x, c);
 }
 
-// Right-hand side at region cell c of S (f_2Dor, or f_2D when DET); R per instance.
-template <bool DET>
-__device__ __forceinline__ void rk_rhs_cell(const RK4Args<float>& A, const float* S, int c, float R, float& fP, float& fW,
-                                            float& fO)
-{
-    const int cn = c - RK_RX, cs = c + RK_RX, cw = c - 1, ce = c + 1;
-    const float* SP = S;
-    const float* SW = S + RK_RN;
-    const float* SO = S + 2 * RK_RN;
-    const float Pc = SP[c], Wc = SW[c], Oc = SO[c];
-    const float upt_num = (A.gmax * Wc) * Pc;
-    const float wk = Wc + A.k1;
-    // two correctly rounded reciprocals instead of three divisions
-    const float iwk = __frcp_rn(wk);
-    const float infil = ((A.alpha * (Pc + A.k2W0)) * __frcp_rn(Pc + A.k2)) * Oc;
-    fP = ((A.cgmax * Wc) * Pc) * iwk;
-    const float upt = upt_num * iwk;
-    const float lapW = add_pow2_times(((SW[cn] + SW[cs]) + SW[cw]) + SW[ce], -4.0f, Wc);
-    const float lapO = add_pow2_times(((SO[cn] + SO[cs]) + SO[cw]) + SO[ce], -4.0f, Oc);
-    if (DET) {
-        const float lapP = add_pow2_times(((SP[cn] + SP[cs]) + SP[cw]) + SP[ce], -4.0f, Pc);
-        fP = (fP - A.d * Pc) + A.DPx * lapP;
-    }
-    fW = ((infil - upt) - A.rW * Wc) + A.DWx * lapW;
-    fO = (R - infil) + A.DOx * lapO;
-}
-
 // One CTA per tile (persistent over tiles).  Stage s (0..3) is evaluated on
 // the region inset by s+1 cells -- exactly the cells whose stage-s value an
 // interior cell depends on -- so the interior is exact after stage 3.  Stage
@@ -86,9 +59,8 @@ __device__ __forceinline__ bool rk_bar_wait(uint32_t bar, uint32_t parity, int l
 
 // The region of tile t (RK_RX columns x ry_n rows of P, W, O, periodic) into X0.  False
 // when its copies did not complete: the instances are flagged and the block returns.
-template <typename T>
-__device__ __forceinline__ bool load_tile(const RK4Args<T>& A, T* X0, int ry_n, const T* __restrict__ P0,
-                                          const T* __restrict__ W0, const T* __restrict__ O0, int L, int x0, int y0, int t,
+__device__ __forceinline__ bool load_tile(const RK4Args<double>& A, double* X0, int ry_n, const double* __restrict__ P0,
+                                          const double* __restrict__ W0, const double* __restrict__ O0, int L, int x0, int y0, int t,
                                           uint32_t bar, uint32_t& phase)
 {
     const int tid = threadIdx.x, rn = RK_RX * ry_n;
@@ -99,8 +71,8 @@ __device__ __forceinline__ bool load_tile(const RK4Args<T>& A, T* X0, int ry_n, 
     // one halo row per thread (3 x ry_n rows): the block takes the bulk path only if
     // every row start is 16-byte aligned
     const int n_rows = 3 * ry_n;
-    const bool shape = (one_wrap && (L * sizeof(T)) % 16 == 0 && x0 >= RK_H && x0 + RK_TX + RK_H <= L) || A.probe_no_copy;
-    const T* src = nullptr;
+    const bool shape = (one_wrap && (L * sizeof(double)) % 16 == 0 && x0 >= RK_H && x0 + RK_TX + RK_H <= L) || A.probe_no_copy;
+    const double* src = nullptr;
     bool aligned = true;
     if (shape && !A.probe_no_copy && tid < n_rows) {
         const int f = tid / ry_n, ry = tid - f * ry_n;
@@ -111,8 +83,8 @@ __device__ __forceinline__ bool load_tile(const RK4Args<T>& A, T* X0, int ry_n, 
     }
     if (shape && __syncthreads_and(aligned)) {
         if (!A.probe_no_copy) {
-            constexpr uint32_t row_bytes = RK_RX * sizeof(T);
-            static_assert((RK_RX * sizeof(float)) % 16 == 0, "bulk rows");
+            constexpr uint32_t row_bytes = RK_RX * sizeof(double);
+            static_assert(row_bytes % 16 == 0, "bulk rows");
             if (tid == 0)
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
                              :: "r"(bar), "r"((uint32_t)n_rows * row_bytes) : "memory");
@@ -155,115 +127,6 @@ __device__ __forceinline__ bool load_tile(const RK4Args<T>& A, T* X0, int ry_n, 
         __syncthreads();
     }
     return true;
-}
-
-template <bool DET>
-__global__ void __launch_bounds__(RK_THREADS, RK_CTAS) rk4_tile_kernel(const RK4Args<float> A)
-{
-    extern __shared__ __align__(16) unsigned char rk_smem[];
-    __shared__ __align__(8) uint64_t tile_bar;
-    float* const X0 = reinterpret_cast<float*>(rk_smem);          // [3][RK_RN] stage-0 input
-    float* const MA = X0 + 3 * RK_RN;                           // [3][RK_RN] stage inputs (ping)
-    float* const MB = MA + 3 * RK_RN;                           // [3][RK_RN] (pong)
-    constexpr int kPer = RK_TX * RK_TY / RK_THREADS;        // interior cells per thread
-    static_assert(RK_TX * RK_TY % RK_THREADS == 0, "interior cells per thread");
-    const int tid = threadIdx.x;
-    const uint32_t bar = rk_saddr(&tile_bar);
-    if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(bar) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-    uint32_t phase = 0;
-    for (int t = blockIdx.x; t < A.n_tasks; t += gridDim.x) {
-        const int4 tk = A.tasks[t];
-        const int k = tk.x;
-        const int L = A.it.L[k];
-        const long long off = A.it.off[k];
-        const long long fs = A.it.fstride[k];
-        const float R = (float)A.it.R[k];
-        const int x0 = tk.y, y0 = tk.z;
-        const float* __restrict__ P0 = (DET ? A.in : A.pstar) + off;
-        const float* __restrict__ W0 = A.in + off + fs;
-        const float* __restrict__ O0 = A.in + off + 2 * fs;
-        if (!load_tile<float>(A, X0, RK_RY, P0, W0, O0, L, x0, y0, t, bar, phase)) return;
-        // Stage s on the region inset by s+1: the 64 x 32 interior with a fixed
-        // thread mapping (kPer cells per thread, whose weighted sums of K stay in
-        // registers), then the ring between the inset and the interior.
-        float acc[3][kPer];
-#pragma unroll
-        for (int s = 0; s < 4; ++s) {
-            const float* S = (s == 0) ? X0 : ((s & 1) ? MA : MB);
-            float* D = (s & 1) ? MB : MA;
-            const float coef = (s == 2) ? A.dt : A.dt2;
-#pragma unroll
-            for (int j = 0; j < kPer; ++j) {
-                const int a = tid + j * RK_THREADS;
-                const int c = ((a / RK_TX) + RK_H) * RK_RX + (a % RK_TX) + RK_H;
-                float k0, k1, k2;
-                rk_rhs_cell<DET>(A, S, c, R, k0, k1, k2);
-                if (s == 0) {
-                    acc[0][j] = k0; acc[1][j] = k1; acc[2][j] = k2;
-                } else if (s == 3) {
-                    acc[0][j] = acc[0][j] + k0; acc[1][j] = acc[1][j] + k1; acc[2][j] = acc[2][j] + k2;
-                } else {
-                    acc[0][j] = add_pow2_times(acc[0][j], 2.0f, k0);
-                    acc[1][j] = add_pow2_times(acc[1][j], 2.0f, k1);
-                    acc[2][j] = add_pow2_times(acc[2][j], 2.0f, k2);
-                }
-                if (s < 3) {
-                    D[c] = X0[c] + coef * k0;
-                    D[RK_RN + c] = X0[RK_RN + c] + coef * k1;
-                    D[2 * RK_RN + c] = X0[2 * RK_RN + c] + coef * k2;
-                }
-            }
-            if (s < 3) {
-                // ring of thickness t = 3 - s: top and bottom bands (t rows of the
-                // inset's width w), then left and right bands (RK_TY rows, t columns)
-                const int in = s + 1, t = 3 - s, w = RK_RX - 2 * in;
-                const int nband = t * w, nside = RK_TY * t;
-                for (int q = tid; q < 2 * nband + 2 * nside; q += RK_THREADS) {
-                    int ry, rx;
-                    if (q < 2 * nband) {
-                        const int qb = q < nband ? q : q - nband;
-                        ry = (q < nband ? in : RK_H + RK_TY) + qb / w;
-                        rx = in + qb % w;
-                    } else {
-                        const int qs = q - 2 * nband;
-                        const int qq = qs < nside ? qs : qs - nside;
-                        ry = RK_H + qq / t;
-                        rx = (qs < nside ? in : RK_H + RK_TX) + qq % t;
-                    }
-                    const int c = ry * RK_RX + rx;
-                    float k0, k1, k2;
-                    rk_rhs_cell<DET>(A, S, c, R, k0, k1, k2);
-                    D[c] = X0[c] + coef * k0;
-                    D[RK_RN + c] = X0[RK_RN + c] + coef * k1;
-                    D[2 * RK_RN + c] = X0[2 * RK_RN + c] + coef * k2;
-                }
-            }
-            __syncthreads();
-        }
-        unsigned st = 0;
-#pragma unroll
-        for (int j = 0; j < kPer; ++j) {
-            const int a = tid + j * RK_THREADS;
-            const int ly = a / RK_TX, lx = a % RK_TX;
-            const int gy = y0 + ly, gx = x0 + lx;
-            if (gy < L && gx < L) {
-                const int c = (ly + RK_H) * RK_RX + lx + RK_H;
-                const long long gi = off + (long long)gy * L + gx;
-#pragma unroll
-                for (int f = 0; f < 3; ++f) {
-                    float v = X0[f * RK_RN + c] + A.dt6 * acc[f][j];
-                    if (v < A.ceps && v >= A.clo) v = 0.0f;
-                    st |= value_status(v);
-                    A.out[gi + f * fs] = v;
-                }
-            }
-        }
-        if (st) atomicOr(A.it.status + k, st);
-    }
 }
 
 // ---- the same step in FP64
@@ -343,7 +206,7 @@ __global__ void __launch_bounds__(RK64_THREADS, 1) rk4_tile64_kernel(const RK4Ar
         const double* __restrict__ P0 = (DET ? A.in : A.pstar) + off;
         const double* __restrict__ W0 = A.in + off + fs;
         const double* __restrict__ O0 = A.in + off + 2 * fs;
-        if (!load_tile<double>(A, X0, ry_n, P0, W0, O0, L, x0, y0, t, bar, phase)) return;
+        if (!load_tile(A, X0, ry_n, P0, W0, O0, L, x0, y0, t, bar, phase)) return;
         double acc[3][kMax];
 #pragma unroll
         for (int j = 0; j < kMax; ++j) acc[0][j] = acc[1][j] = acc[2][j] = 0.0;
@@ -427,24 +290,6 @@ __global__ void __launch_bounds__(RK64_THREADS, 1) rk4_tile64_kernel(const RK4Ar
         }
         if (st) atomicOr(A.it.status + k, st);
     }
-}
-
-template <>
-cudaError_t launch_rk4<float>(const RK4Args<float>& a, bool det, int grid, cudaStream_t s)
-{
-    if (a.n_tasks <= 0) return cudaSuccess;
-    const size_t smem = 9 * (size_t)RK_RN * sizeof(float);
-    static bool attr[2] = {false, false};
-    if (!attr[det ? 1 : 0]) {
-        const cudaError_t e =
-            det ? cudaFuncSetAttribute(rk4_tile_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                : cudaFuncSetAttribute(rk4_tile_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        attr[det ? 1 : 0] = true;
-    }
-    if (det) rk4_tile_kernel<true><<<grid, RK_THREADS, smem, s>>>(a);
-    else rk4_tile_kernel<false><<<grid, RK_THREADS, smem, s>>>(a);
-    return cudaGetLastError();
 }
 
 template <>
