@@ -319,6 +319,17 @@ TM_HD bool is_zero(double x) { return (f64_bits(x) << 1) == 0; }
 // The sign by its bit (the compiler's own negation and absolute value are FP64 additions).
 TM_HD double abs_bits(double x) { return bits_f64(f64_bits(x) & ~kSign); }
 TM_HD double with_sign(double x, bool negative) { return bits_f64((f64_bits(x) & ~kSign) | (negative ? kSign : 0)); }
+// a < b by the hardware's comparison, kept behind the caller's branch.
+TM_HD bool hw_less(double a, double b)
+{
+#ifdef __CUDA_ARCH__
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.lt.f64 p, %1, %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r) : "d"(a), "d"(b));
+    return r != 0;
+#else
+    return a < b;
+#endif
+}
 // x in [lo, hi) by the hardware's comparisons, kept behind the caller's branch.
 TM_HD bool hw_in_range(double x, double lo, double hi)
 {
