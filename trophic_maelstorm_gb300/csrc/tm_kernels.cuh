@@ -14,6 +14,30 @@ struct tm_ctx {
 
 namespace tmg {
 
+// Programmatic dependent launch: a kernel launched by launch_pdl may start while its
+// predecessor on the stream still runs, and waits for the predecessor's end (and its
+// writes) in pdl_wait(), which every such kernel calls before it touches memory that
+// another kernel writes.  Its prologue -- tables, barriers, the launch itself -- then
+// overlaps the predecessor's tail.  pdl_trigger() lets the successor start.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... Params, typename... Args>
+cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, const Args&... args)
+{
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute a;
+    a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &a;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, static_cast<Params>(args)...);
+}
+
 // Dornic constants of one instance: lambda e^{beta dt}, 1/lambda, e^{beta dt}, (e^{beta dt}-1)/beta
 struct __align__(16) Dc4 { double x, y, z, w; };
 

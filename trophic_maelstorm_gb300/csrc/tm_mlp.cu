@@ -4,10 +4,10 @@
 // The reference has no learned part; the network, its rounding points and its
 // optimiser are specified in include/tm.h (tm_mlp_*).  One CTA owns a tile of
 // 128 samples (sample t = TMEM lane t) and runs the whole forward and backward
-// pass of that tile with 16 warps: warp w reads TMEM lane quarter w % 4 (the
+// pass of that tile with 32 warps: warp w reads TMEM lane quarter w % 4 (the
 // quarter a warp may access) and handles column slice w / 4, so a thread does
-// 32 of the 128 columns of its sample and the 128-sample column sums are split
-// four ways:
+// 16 of the 128 columns of its sample; sums over 128 columns or samples are formed
+// from four parts of 32 terms:
 //   * the two 128x128 layers and the four GEMMs of their backward pass are
 //     tcgen05.mma (kind::f16, BF16 x BF16 -> FP32, M = N = K = 128), issued by
 //     one thread, with both operands in shared memory in the K-major
@@ -18,6 +18,13 @@
 //   * each CTA writes its partial gradient; a second kernel sums the partials
 //     in tile order (no atomics: the result does not depend on scheduling) and
 //     applies Adam to the FP32 master weights, refreshing their BF16 copies.
+// Bound by one tile's serial chain (phases of a few thousand cycles between barriers), not
+// by arithmetic: 12,000 samples are 94 tiles on 152 SMs.  Measured per training step:
+// 53.3 us with everything unrolled (waiting for instructions), tanh evaluated twice and
+// 2-byte transposed stores; 36.4 us with loops, gelu' kept in TMEM, matrix-load
+// transposes, 16-byte constant loads, one polling warp, and both kernels' prologues overlapping
+// their predecessors (programmatic dependent launch: 43 -> 36).  512 or 1024 threads made
+// no difference before the shared-memory work went down.
 // Every wait on an MMA completion is bounded: on timeout the CTA records an
 // error, waits once more (again bounded) for the MMAs it issued, frees its
 // TMEM and returns; the update kernel then leaves the parameters unchanged.
@@ -34,12 +41,14 @@
 namespace {
 
 constexpr int TS = 128;              // samples per tile = TMEM lanes
-constexpr int NT = 512;              // threads per CTA: 4 column slices x 128 samples
-constexpr int NS = NT / TS;          // column slices (32 columns each)
+constexpr int NT = 1024;             // threads per CTA: 8 column slices x 128 samples
+constexpr int CW = 128 / (NT / TS);  // columns of a thread's slice
+constexpr int NS = 4;                // parts of 32 terms that each sum over 128 is formed from
 constexpr int OFF_W1 = 0, OFF_B1 = 384, OFF_W2 = 512, OFF_B2 = 16896, OFF_W3 = 17024, OFF_B3 = 33408,
               OFF_W4 = 33536, OFF_B4 = 33792, NP = 33794;
 static_assert(NP == TM_MLP_NPARAMS, "parameter layout");
-constexpr int PS = 33808;            // per-tile stride of the partial gradients (16-byte aligned rows)
+constexpr int PS = 33808;            // per-tile stride of the partial gradients (rows stay 32-byte aligned)
+static_assert(PS % 8 == 0 && OFF_W2 % 8 == 0 && OFF_W3 % 8 == 0, "32-byte aligned gradient rows");
 
 // shared memory map
 constexpr int BUF = 32768;           // one 128 x 128 BF16 operand tile
@@ -120,22 +129,26 @@ __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, int limi
     return false;
 }
 
-// 32 consecutive FP32 columns of this thread's TMEM lane
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v)
+// 8 consecutive FP32 columns of this thread's TMEM lane
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v)
 {
-    uint32_t r[32];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                 "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-                 "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-                   "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]),
-                   "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]),
-                   "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                  : "r"(taddr));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const float* v)
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                 :: "r"(taddr), "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])),
+                    "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])),
+                    "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7]))
+                 : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
 __device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
@@ -153,6 +166,14 @@ __device__ __forceinline__ float gelu_grad(float a)
 {
     const float th = tanhf(kGeluC * (a + kGeluK * (a * a * a)));
     return 0.5f * (1.0f + th) + 0.5f * a * (1.0f - th * th) * kGeluC * (1.0f + 3.0f * kGeluK * (a * a));
+}
+
+// both from one tanh
+__device__ __forceinline__ float gelu_and_grad(float a, float& grad)
+{
+    const float th = tanhf(kGeluC * (a + kGeluK * (a * a * a)));
+    grad = 0.5f * (1.0f + th) + 0.5f * a * (1.0f - th * th) * kGeluC * (1.0f + 3.0f * kGeluK * (a * a));
+    return 0.5f * a * (1.0f + th);
 }
 
 // 128 x 128 BF16 row-major matrix (global) -> K-major core-matrix tile (shared)
@@ -180,9 +201,49 @@ __device__ __forceinline__ void store8(unsigned char* buf, int r, int k0, const 
     *reinterpret_cast<uint4*>(buf + cm(r, k0)) = *reinterpret_cast<const uint4*>(h);
 }
 
-__device__ __forceinline__ void store1(unsigned char* buf, int r, int k, __nv_bfloat16 h)
+// The transpose of a warp's 32 rows x CW columns (rows r0.., columns k0.. of `from`, just
+// stored by this warp) into rows k0.., columns r0.. of `to`: an 8 x 8 block is 128
+// contiguous bytes in either tile, so four blocks go by one transposing matrix load and
+// one matrix store (2-byte stores took 4 bank cycles each, 16 of them a thread).
+__device__ __forceinline__ void transpose_warp(const unsigned char* from, unsigned char* to, int r0, int k0)
 {
-    *reinterpret_cast<__nv_bfloat16*>(buf + cm(r, k)) = h;
+    const int lane = threadIdx.x & 31, blk = lane >> 3, i = lane & 7;
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < CW; c += 8) {
+        uint32_t m0, m1, m2, m3;
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(m0), "=r"(m1), "=r"(m2), "=r"(m3) : "r"(saddr(from + cm(r0 + blk * 8 + i, k0 + c))) : "memory");
+        asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};"
+                     :: "r"(saddr(to + cm(k0 + c + i, r0 + blk * 8))), "r"(m0), "r"(m1), "r"(m2), "r"(m3) : "memory");
+    }
+}
+
+// 8 consecutive floats of shared memory (16-byte aligned)
+__device__ __forceinline__ void lds8(const float* p, float* v)
+{
+    const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+
+// 8 floats to a 32-byte aligned global address in one instruction
+__device__ __forceinline__ void stg8(float* p, const float* v)
+{
+    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                 :: "l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
+}
+
+// z1 = W1 x + b1 of columns j .. j + 7 (j a multiple of 8)
+__device__ __forceinline__ void layer1(const float* W1s, const float* bs, int j, float x0, float x1, float x2, float* z)
+{
+    float w[24], b[8];
+    lds8(W1s + 3 * j, w);
+    lds8(W1s + 3 * j + 8, w + 8);
+    lds8(W1s + 3 * j + 16, w + 16);
+    lds8(bs + j, b);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) z[i] = ((w[3 * i] * x0 + w[3 * i + 1] * x1) + w[3 * i + 2] * x2) + b[i];
 }
 
 struct MlpArgs {
@@ -226,20 +287,15 @@ __global__ void __launch_bounds__(NT, 1) mlp_tile_kernel(MlpArgs a)
     const int tid = threadIdx.x, warp = tid >> 5;
     const int q = warp & 3, cs = warp >> 2;            // TMEM lane quarter, column slice
     const int t = q * 32 + (tid & 31);                 // this thread's sample (= TMEM lane)
-    const int c0 = cs * 32;                            // first column of this thread's slice
+    const int c0 = cs * CW;                            // first column of this thread's slice
+    const int up = tid >> 9, sj = tid & 127, sp = (tid >> 7) & 3;   // sums: half of the block, row or column, part
     const int tile = blockIdx.x;
     const long long s = (long long)tile * TS + t;
     const bool valid = s < a.n;
     const uint32_t bar_a = saddr(bar);
 
-    for (int i = tid; i < 384; i += NT) W1s[i] = bf16r(a.p[OFF_W1 + i]);
-    for (int i = tid; i < 128; i += NT) {
-        bs[i] = a.p[OFF_B1 + i];
-        bs[128 + i] = a.p[OFF_B2 + i];
-        bs[256 + i] = a.p[OFF_B3 + i];
-    }
-    for (int i = tid; i < 256; i += NT) W4s[i] = bf16r(a.p[OFF_W4 + i]);
-    if (tid < 2) b4s[tid] = a.p[OFF_B4 + tid];
+    // what the update kernel does not write comes before the wait for it
+    tmg::pdl_trigger();
     float x0 = 0.0f, x1 = 0.0f, x2 = 0.0f;
     if (valid) {
         x0 = a.x[3 * s];
@@ -251,8 +307,6 @@ __global__ void __launch_bounds__(NT, 1) mlp_tile_kernel(MlpArgs a)
         xs[3 * t + 1] = x1;
         xs[3 * t + 2] = x2;
     }
-    load_tile(B0, a.W2);
-    load_tile(B1, a.W3);
     if (tid == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(bar_a) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -262,6 +316,17 @@ __global__ void __launch_bounds__(NT, 1) mlp_tile_kernel(MlpArgs a)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    tmg::pdl_wait();
+    load_tile(B0, a.W2);
+    load_tile(B1, a.W3);
+    for (int i = tid; i < 384; i += NT) W1s[i] = bf16r(a.p[OFF_W1 + i]);
+    for (int i = tid; i < 128; i += NT) {
+        bs[i] = a.p[OFF_B1 + i];
+        bs[128 + i] = a.p[OFF_B2 + i];
+        bs[256 + i] = a.p[OFF_B3 + i];
+    }
+    for (int i = tid; i < 256; i += NT) W4s[i] = bf16r(a.p[OFF_W4 + i]);
+    if (tid < 2) b4s[tid] = a.p[OFF_B4 + tid];
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -271,21 +336,22 @@ __global__ void __launch_bounds__(NT, 1) mlp_tile_kernel(MlpArgs a)
     uint32_t phase = 0;
     bool failed = false;
     __align__(16) __nv_bfloat16 hb[8];
-    float v[32];
+    float v[8], dg[8], cv[8];
+    // The passes over a thread's columns take 8 at a time in loops that stay loops: a
+    // CTA runs this code once, so what it waited for most was instructions (4.6 of 12
+    // stall cycles per issue with everything unrolled).
 
     do {
         // ---- layer 1 (CUDA cores): h1 = bf16(gelu(W1 x + b1)) -> B2 (A operand); h1^T -> B3
+#pragma unroll 1
+        for (int g = 0; g < CW / 8; ++g) {
+            const int j = c0 + g * 8;
+            layer1(W1s, bs, j, x0, x1, x2, v);
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int j = c0 + g * 8 + i;
-                const float z = ((W1s[3 * j] * x0 + W1s[3 * j + 1] * x1) + W1s[3 * j + 2] * x2) + bs[j];
-                hb[i] = __float2bfloat16_rn(gelu(z));
-                if (TRAIN) store1(B3, j, t, hb[i]);
-            }
-            store8(B2, t, c0 + g * 8, hb);
+            for (int i = 0; i < 8; ++i) hb[i] = __float2bfloat16_rn(gelu(v[i]));
+            store8(B2, t, j, hb);
         }
+        if (TRAIN) transpose_warp(B2, B3, q * 32, c0);
         fence_async_smem();
         __syncthreads();
         if (tid == 0 && !a.probe_no_mma) {
@@ -293,23 +359,26 @@ __global__ void __launch_bounds__(NT, 1) mlp_tile_kernel(MlpArgs a)
             mma_128(tmem + 0, saddr(B2), saddr(B0));          // a2 - b2 -> TMEM cols 0..127
             mma_commit(bar_a);
         }
-        failed = __syncthreads_or(!bar_wait(bar_a, phase, a.wait_limit));
+        failed = __syncthreads_or(warp == 0 && !bar_wait(bar_a, phase, a.wait_limit));
         phase ^= 1;
         if (failed) break;
         tc_fence_after();
 
-        // ---- layer 2 epilogue: h2 = bf16(gelu(a2)) -> B2 (A operand); h2^T -> B4
-        tmem_ld32(lane + 0, v);
-#pragma unroll
-        for (int g = 0; g < 4; ++g) {
+        // ---- layer 2 epilogue: h2 = bf16(gelu(a2)) -> B2 (A operand); h2^T -> B4;
+        //      gelu'(a2) takes the place of a2 - b2 in TMEM
+#pragma unroll 1
+        for (int g = 0; g < CW / 8; ++g) {
+            tmem_ld8(lane + g * 8, v);
+            lds8(bs + 128 + c0 + g * 8, cv);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                const int j = c0 + g * 8 + i;
-                hb[i] = __float2bfloat16_rn(gelu(v[g * 8 + i] + bs[128 + j]));
-                if (TRAIN) store1(B4, j, t, hb[i]);
+                const float z = v[i] + cv[i];
+                hb[i] = __float2bfloat16_rn(TRAIN ? gelu_and_grad(z, dg[i]) : gelu(z));
             }
             store8(B2, t, c0 + g * 8, hb);
+            if (TRAIN) tmem_st8(lane + g * 8, dg);
         }
+        if (TRAIN) transpose_warp(B2, B4, q * 32, c0);
         fence_async_smem();
         tc_fence_before();
         __syncthreads();
@@ -318,26 +387,35 @@ __global__ void __launch_bounds__(NT, 1) mlp_tile_kernel(MlpArgs a)
             mma_128(tmem + 128, saddr(B2), saddr(B1));        // a3 - b3 -> TMEM cols 128..255
             mma_commit(bar_a);
         }
-        failed = __syncthreads_or(!bar_wait(bar_a, phase, a.wait_limit));
+        failed = __syncthreads_or(warp == 0 && !bar_wait(bar_a, phase, a.wait_limit));
         phase ^= 1;
         if (failed) break;
         tc_fence_after();
 
-        // ---- layer 3 epilogue and output layer: y = W4 gelu(a3) + b4, slice partials summed in
-        //      slice order (h3 kept FP32 in F for dW4)
-        {
-            float y0 = 0.0f, y1 = 0.0f;
-            tmem_ld32(lane + 128, v);
+        // ---- layer 3 epilogue and output layer: y = W4 gelu(a3) + b4, h3 in FP32 in F (also for
+        //      dW4), in four parts of 32 columns summed in order
+#pragma unroll 1
+        for (int g = 0; g < CW / 8; ++g) {
+            tmem_ld8(lane + 128 + g * 8, v);
+            lds8(bs + 256 + c0 + g * 8, cv);
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-                const int j = c0 + i;
-                const float h = gelu(v[i] + bs[256 + j]);
-                y0 = y0 + W4s[j] * h;
-                y1 = y1 + W4s[128 + j] * h;
-                if (TRAIN) F[j * FPAD + t] = h;
+            for (int i = 0; i < 8; ++i) {
+                const float z = v[i] + cv[i];
+                F[(c0 + g * 8 + i) * FPAD + t] = TRAIN ? gelu_and_grad(z, dg[i]) : gelu(z);
             }
-            red[(cs * TS + t) * 3] = y0;
-            red[(cs * TS + t) * 3 + 1] = y1;
+            if (TRAIN) tmem_st8(lane + 128 + g * 8, dg);     // gelu'(a3)
+        }
+        __syncthreads();
+        {
+            // output `up` of sample sj over columns 32 sp .. 32 sp + 31
+            float y = 0.0f;
+#pragma unroll 1
+            for (int j = 32 * sp; j < 32 * sp + 32; j += 8) {
+                lds8(W4s + 128 * up + j, cv);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) y = y + cv[i] * F[(j + i) * FPAD + sj];
+            }
+            red[(sp * TS + sj) * 3 + up] = y;
         }
         __syncthreads();
         float dy0 = 0.0f, dy1 = 0.0f;
@@ -373,16 +451,11 @@ __global__ void __launch_bounds__(NT, 1) mlp_tile_kernel(MlpArgs a)
         dy0 = dys[2 * t];
         dy1 = dys[2 * t + 1];
         {
-            // gW4[o][j] = sum_u dy_o[u] h3[u][j]: thread (j = tid & 127, part p = tid >> 7) sums 32 samples
-            const int j = tid & 127, p = tid >> 7;
-            float g0 = 0.0f, g1 = 0.0f;
-            for (int u = 32 * p; u < 32 * p + 32; ++u) {
-                const float h = F[j * FPAD + u];
-                g0 = g0 + dys[2 * u] * h;
-                g1 = g1 + dys[2 * u + 1] * h;
-            }
-            red[(p * TS + j) * 3] = g0;
-            red[(p * TS + j) * 3 + 1] = g1;
+            // gW4[o][j] = sum_u dy_o[u] h3[u][j]: output `up`, column sj, samples 32 sp ..
+            float g = 0.0f;
+#pragma unroll 8
+            for (int u = 32 * sp; u < 32 * sp + 32; ++u) g = g + dys[2 * u + up] * F[sj * FPAD + u];
+            red[(sp * TS + sj) * 3 + up] = g;
         }
         __syncthreads();
         if (tid < 128) {
@@ -394,33 +467,33 @@ __global__ void __launch_bounds__(NT, 1) mlp_tile_kernel(MlpArgs a)
             gp[OFF_W4 + tid] = g0;
             gp[OFF_W4 + 128 + tid] = g1;
         }
-        if (tid == 0) {
-            float s0 = 0.0f, s1 = 0.0f, sl = 0.0f;
-            for (int u = 0; u < TS; ++u) {
-                s0 = s0 + dys[2 * u];
-                s1 = s1 + dys[2 * u + 1];
-                sl = sl + ls[u];
-            }
-            gp[OFF_B4] = s0;
-            gp[OFF_B4 + 1] = s1;
-            a.loss_part[tile] = sl * a.inv_norm;
+        // the three sums over samples, in sample order, on three other warps
+        if (tid == 128 || tid == 160 || tid == 192) {
+            const float* from = tid == 128 ? dys : (tid == 160 ? dys + 1 : ls);
+            const int step = tid == 192 ? 1 : 2;
+            float sum = 0.0f;
+#pragma unroll 16
+            for (int u = 0; u < TS; ++u) sum = sum + from[step * u];
+            if (tid == 192) a.loss_part[tile] = sum * a.inv_norm;
+            else gp[OFF_B4 + (tid == 160)] = sum;
         }
         __syncthreads();                                      // F (B0..B2) and red free again
 
         // ---- dz3 = bf16((dy W4) * gelu'(a3)) -> B2 (A operand of dH2); dz3^T -> B5 (A operand of dW3)
         load_tile(B1, a.W3T);
-        tmem_ld32(lane + 128, v);
-#pragma unroll
-        for (int g = 0; g < 4; ++g) {
+#pragma unroll 1
+        for (int g = 0; g < CW / 8; ++g) {
+            tmem_ld8(lane + 128 + g * 8, dg);
+            lds8(W4s + c0 + g * 8, cv);
+            lds8(W4s + 128 + c0 + g * 8, v);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                const int j = c0 + g * 8 + i;
-                const float dh = dy0 * W4s[j] + dy1 * W4s[128 + j];
-                hb[i] = __float2bfloat16_rn(dh * gelu_grad(v[g * 8 + i] + bs[256 + j]));
-                store1(B5, j, t, hb[i]);
+                const float dh = dy0 * cv[i] + dy1 * v[i];
+                hb[i] = __float2bfloat16_rn(dh * dg[i]);
             }
             store8(B2, t, c0 + g * 8, hb);
         }
+        transpose_warp(B2, B5, q * 32, c0);
         fence_async_smem();
         tc_fence_before();
         __syncthreads();
@@ -430,8 +503,8 @@ __global__ void __launch_bounds__(NT, 1) mlp_tile_kernel(MlpArgs a)
             mma_128(tmem + 384, saddr(B5), saddr(B4));        // gW3 = dz3^T h2    -> cols 384..511
             mma_commit(bar_a);
         }
-        red[(cs * TS + t) * 3 + 2] = row_sum_part(B5, t, cs);   // gb3 partial: row t of dz3^T, samples 32 cs..
-        failed = __syncthreads_or(!bar_wait(bar_a, phase, a.wait_limit));
+        if (up == 0) red[(sp * TS + sj) * 3 + 2] = row_sum_part(B5, sj, sp);   // gb3 partial: row sj of dz3^T, samples 32 sp..
+        failed = __syncthreads_or(warp == 0 && !bar_wait(bar_a, phase, a.wait_limit));
         phase ^= 1;
         if (failed) break;
         tc_fence_after();
@@ -443,27 +516,17 @@ __global__ void __launch_bounds__(NT, 1) mlp_tile_kernel(MlpArgs a)
 
         // ---- gW3 rows; dz2 = bf16(dH2 * gelu'(a2)) -> B2; dz2^T -> B5
         load_tile(B0, a.W2T);
-        tmem_ld32(lane + 384, v);
-        {
-            float4* dst = reinterpret_cast<float4*>(gp + OFF_W3 + t * 128 + c0);
+#pragma unroll 1
+        for (int g = 0; g < CW / 8; ++g) {
+            tmem_ld8(lane + 384 + g * 8, v);
+            stg8(gp + OFF_W3 + t * 128 + c0 + g * 8, v);
+            tmem_ld8(lane + 256 + g * 8, v);
+            tmem_ld8(lane + g * 8, dg);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+            for (int i = 0; i < 8; ++i) hb[i] = __float2bfloat16_rn(v[i] * dg[i]);
+            store8(B2, t, c0 + g * 8, hb);
         }
-        {
-            float z[32];
-            tmem_ld32(lane + 256, v);
-            tmem_ld32(lane + 0, z);
-    #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const int j = c0 + g * 8 + i;
-                    hb[i] = __float2bfloat16_rn(v[g * 8 + i] * gelu_grad(z[g * 8 + i] + bs[128 + j]));
-                    store1(B5, j, t, hb[i]);
-                }
-                store8(B2, t, c0 + g * 8, hb);
-            }
-        }
+        transpose_warp(B2, B5, q * 32, c0);
         fence_async_smem();
         tc_fence_before();
         __syncthreads();                                      // also: every gb3 read of red is done
@@ -473,8 +536,8 @@ __global__ void __launch_bounds__(NT, 1) mlp_tile_kernel(MlpArgs a)
             mma_128(tmem + 0, saddr(B5), saddr(B3));          // gW2 = dz2^T h1    -> cols 0..127
             mma_commit(bar_a);
         }
-        red[(cs * TS + t) * 3 + 2] = row_sum_part(B5, t, cs);   // gb2 partial
-        failed = __syncthreads_or(!bar_wait(bar_a, phase, a.wait_limit));
+        if (up == 0) red[(sp * TS + sj) * 3 + 2] = row_sum_part(B5, sj, sp);   // gb2 partial
+        failed = __syncthreads_or(warp == 0 && !bar_wait(bar_a, phase, a.wait_limit));
         phase ^= 1;
         if (failed) break;
         tc_fence_after();
@@ -485,46 +548,45 @@ __global__ void __launch_bounds__(NT, 1) mlp_tile_kernel(MlpArgs a)
         }
 
         // ---- gW2 rows; dz1 = dH1 * gelu'(z1) (FP32) -> F; gW1, gb1 by column sums
-        tmem_ld32(lane + 0, v);
-        {
-            float4* dst = reinterpret_cast<float4*>(gp + OFF_W2 + t * 128 + c0);
+#pragma unroll 1
+        for (int g = 0; g < CW / 8; ++g) {
+            tmem_ld8(lane + g * 8, v);
+            stg8(gp + OFF_W2 + t * 128 + c0 + g * 8, v);
+            tmem_ld8(lane + 128 + g * 8, v);
+            layer1(W1s, bs, c0 + g * 8, x0, x1, x2, dg);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-        }
-        tmem_ld32(lane + 128, v);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-            const int j = c0 + i;
-            const float z = ((W1s[3 * j] * x0 + W1s[3 * j + 1] * x1) + W1s[3 * j + 2] * x2) + bs[j];
-            F[j * FPAD + t] = v[i] * gelu_grad(z);
+            for (int i = 0; i < 8; ++i) F[(c0 + g * 8 + i) * FPAD + t] = v[i] * gelu_grad(dg[i]);
         }
         __syncthreads();                                      // F complete; every gb2 read of red is done
         {
-            const int j = tid & 127, p = tid >> 7;
-            float g0 = 0.0f, g1 = 0.0f, g2 = 0.0f;
-            for (int u = 32 * p; u < 32 * p + 32; ++u) {
-                const float d = F[j * FPAD + u];
-                g0 = g0 + d * xs[3 * u];
-                g1 = g1 + d * xs[3 * u + 1];
-                g2 = g2 + d * xs[3 * u + 2];
+            // gW1[j][k] = sum_u dz1[u][j] x[u][k], k = 0, 1 by the lower half, 2 by the upper
+            float g0 = 0.0f, g1 = 0.0f;
+#pragma unroll 8
+            for (int u = 32 * sp; u < 32 * sp + 32; ++u) {
+                const float d = F[sj * FPAD + u];
+                g0 = g0 + d * xs[3 * u + 2 * up];
+                if (up == 0) g1 = g1 + d * xs[3 * u + 1];
             }
-            red[(p * TS + j) * 3] = g0;
-            red[(p * TS + j) * 3 + 1] = g1;
-            red[(p * TS + j) * 3 + 2] = g2;
+            red[(sp * TS + sj) * 3 + 2 * up] = g0;
+            if (up == 0) red[(sp * TS + sj) * 3 + 1] = g1;
+        }
+        if (tid >= NT - 128) {                                // gb1, in sample order
+            float gb = 0.0f;
+#pragma unroll 16
+            for (int u = 0; u < TS; ++u) gb = gb + F[sj * FPAD + u];
+            gp[OFF_B1 + sj] = gb;
         }
         __syncthreads();
         if (tid < 128) {
-            float g0 = 0.0f, g1 = 0.0f, g2 = 0.0f, gb = 0.0f;
+            float g0 = 0.0f, g1 = 0.0f, g2 = 0.0f;
             for (int p = 0; p < NS; ++p) {
                 g0 = g0 + red[(p * TS + tid) * 3];
                 g1 = g1 + red[(p * TS + tid) * 3 + 1];
                 g2 = g2 + red[(p * TS + tid) * 3 + 2];
             }
-            for (int u = 0; u < TS; ++u) gb = gb + F[tid * FPAD + u];
             gp[OFF_W1 + 3 * tid] = g0;
             gp[OFF_W1 + 3 * tid + 1] = g1;
             gp[OFF_W1 + 3 * tid + 2] = g2;
-            gp[OFF_B1 + tid] = gb;
         }
     } while (false);
 
@@ -556,18 +618,60 @@ struct AdamArgs {
     const int* err;                  // a tile kernel's wait ran out: the partials are invalid, change nothing
 };
 
-__global__ void mlp_adam_kernel(AdamArgs a)
+// A block's 64 parameters: its 256 threads bring 128 tiles' partials into shared memory
+// at a time, all loads in flight together, and one thread per parameter adds them in
+// tile order.  (One thread per parameter loading its own 94 partials waited for memory
+// six times over: 9.6 us, 7.3 now, the serial FP64 loss sum included.)
+constexpr int kAdamParams = 64, kAdamThreads = 256, kAdamTiles = 128;
+constexpr int kAdamGrid = (NP + kAdamParams - 1) / kAdamParams + 1;      // the last block sums the loss
+
+__global__ void __launch_bounds__(kAdamThreads) mlp_adam_kernel(AdamArgs a)
 {
+    __shared__ float part[kAdamTiles][kAdamParams];
+    tmg::pdl_trigger();
+    tmg::pdl_wait();
     if (a.err != nullptr && *a.err != 0) return;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < NP; i += gridDim.x * blockDim.x) {
-        float pv = a.p[i];
+    const int tid = threadIdx.x;
+    if (blockIdx.x == gridDim.x - 1) {
+        // FP64 sum of the FP32 losses: lanes take every 32nd tile, then a butterfly
+        if (a.loss_out && tid < 32) {
+            double sl = 0.0;
+            for (int k = tid; k < a.n_tiles; k += 32) sl += (double)a.loss_part[k];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) sl += __shfl_xor_sync(0xffffffffu, sl, o);
+            if (tid == 0) *a.loss_out = sl;
+        }
+        return;
+    }
+    const int p0 = blockIdx.x * kAdamParams, i = p0 + tid;
+    float g = 0.0f, pv = 0.0f, m0 = 0.0f, v0 = 0.0f;
+    if (tid < kAdamParams && i < NP) {
+        pv = a.p[i];
+        if (a.update) {
+            m0 = a.m[i];
+            v0 = a.v[i];
+        }
+    }
+    for (int k0 = 0; k0 < a.n_tiles; k0 += kAdamTiles) {
+        const int nk = min(kAdamTiles, a.n_tiles - k0);
+        const int c = tid % kAdamParams;
+        if (k0 > 0) __syncthreads();
+        // PS > NP: the columns beyond the last parameter are allocated, and not used
+#pragma unroll 16
+        for (int k = tid / kAdamParams; k < nk; k += kAdamThreads / kAdamParams)
+            part[k][c] = p0 + c < PS ? a.part[(size_t)(k0 + k) * PS + p0 + c] : 0.0f;
+        __syncthreads();
+        if (tid < kAdamParams) {
+#pragma unroll 16
+            for (int k = 0; k < nk; ++k) g = g + part[k][tid];
+        }
+    }
+    if (tid < kAdamParams && i < NP) {
         if (a.n_tiles > 0) {
-            float g = 0.0f;
-            for (int k = 0; k < a.n_tiles; ++k) g = g + a.part[(size_t)k * PS + i];
             if (a.grad_out) a.grad_out[i] = g;
             if (a.update) {
-                const float mv = a.b1 * a.m[i] + (1.0f - a.b1) * g;
-                const float vv = a.b2 * a.v[i] + (1.0f - a.b2) * (g * g);
+                const float mv = a.b1 * m0 + (1.0f - a.b1) * g;
+                const float vv = a.b2 * v0 + (1.0f - a.b2) * (g * g);
                 pv = pv - a.lr * (mv * a.c1) / (sqrtf(vv * a.c2) + a.eps);
                 a.m[i] = mv;
                 a.v[i] = vv;
@@ -585,11 +689,6 @@ __global__ void mlp_adam_kernel(AdamArgs a)
             a.W3[r * 128 + c] = h;
             a.W3T[c * 128 + r] = h;
         }
-    }
-    if (a.loss_out && blockIdx.x == 0 && threadIdx.x == 0) {
-        double sl = 0.0;
-        for (int k = 0; k < a.n_tiles; ++k) sl += (double)a.loss_part[k];
-        *a.loss_out = sl;
     }
 }
 
@@ -644,6 +743,11 @@ int grow_tiles(tm_mlp* m, int tiles)
     }
     m->tiles_cap = tiles;
     return TM_OK;
+}
+
+void launch_adam(const AdamArgs& a, cudaStream_t s)
+{
+    (void)tmg::launch_pdl(mlp_adam_kernel, dim3(kAdamGrid), dim3(kAdamThreads), 0, s, a);   // finish() reports errors
 }
 
 cudaError_t set_smem_attr()
@@ -723,7 +827,7 @@ int upload_params(tm_mlp* m, const float* params)
     MLP_CUDA(cudaMemsetAsync(m->m, 0, NP * sizeof(float), s));
     MLP_CUDA(cudaMemsetAsync(m->v, 0, NP * sizeof(float), s));
     AdamArgs a = adam_args(m, 0, nullptr, nullptr, 0, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f);
-    mlp_adam_kernel<<<(NP + 255) / 256, 256, 0, s>>>(a);
+    launch_adam(a, s);
     m->step = 0;
     return finish(m);
 }
@@ -827,9 +931,9 @@ int tm_mlp_loss_grad(tm_mlp* m, float inv_norm, double* loss, float* grad)
     }
     cudaStream_t s = m->ctx->stream;
     const int tiles = (m->n + TS - 1) / TS;
-    mlp_tile_kernel<true><<<tiles, NT, SM_TOTAL, s>>>(tile_args(m, m->x, m->n, inv_norm, nullptr));
+    (void)tmg::launch_pdl(mlp_tile_kernel<true>, dim3(tiles), dim3(NT), SM_TOTAL, s, tile_args(m, m->x, m->n, inv_norm, nullptr));
     AdamArgs a = adam_args(m, tiles, m->loss_dev, m->grad, 0, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f);
-    mlp_adam_kernel<<<(NP + 255) / 256, 256, 0, s>>>(a);
+    launch_adam(a, s);
     const int rc = finish(m);
     if (rc != TM_OK) return rc;
     if (grad) MLP_CUDA(cudaMemcpy(grad, m->grad, NP * sizeof(float), cudaMemcpyDeviceToHost));
@@ -857,9 +961,9 @@ int tm_mlp_train(tm_mlp* m, int steps, float lr, float beta1, float beta2, float
         const long long st = m->step + 1 + k;
         const float c1 = (float)(1.0 / (1.0 - std::pow((double)beta1, (double)st)));
         const float c2 = (float)(1.0 / (1.0 - std::pow((double)beta2, (double)st)));
-        mlp_tile_kernel<true><<<tiles, NT, SM_TOTAL, s>>>(tile_args(m, m->x, m->n, inv_norm, nullptr));
+        (void)tmg::launch_pdl(mlp_tile_kernel<true>, dim3(tiles), dim3(NT), SM_TOTAL, s, tile_args(m, m->x, m->n, inv_norm, nullptr));
         AdamArgs a = adam_args(m, tiles, m->loss_dev + k, nullptr, 1, lr, beta1, beta2, eps, c1, c2);
-        mlp_adam_kernel<<<(NP + 255) / 256, 256, 0, s>>>(a);
+        launch_adam(a, s);
     }
     const int rc = finish(m);
     if (rc != TM_OK) return rc;
