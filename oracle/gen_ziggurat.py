@@ -75,9 +75,9 @@ def emit():
         fh.write("#pragma once\n#include <stdint.h>\nnamespace tmg {\n")
         fh.write(f"constexpr int kZigN = {N};\nconstexpr int kZigBits = {BITS};\n")
         fh.write(f"constexpr double kZigR = {float(R).hex()};\n")
-        fh.write(f"__device__ const uint32_t kZigK[{N}] = {{{kl}}};\n")
-        fh.write(f"__device__ const double kZigW[{N}] = {{{wl}}};\n")
-        fh.write(f"__device__ const double kZigF[{N + 1}] = {{{fl}}};\n")
+        fh.write(f"constexpr uint32_t kZigK[{N}] = {{{kl}}};\n")
+        fh.write(f"constexpr double kZigW[{N}] = {{{wl}}};\n")
+        fh.write(f"constexpr double kZigF[{N + 1}] = {{{fl}}};\n")
         fh.write("}  // namespace tmg\n")
 
 

@@ -290,7 +290,7 @@ RK4Args<T> rk4_args(const tm_batch* b, const T* in, const T* pstar, T* out)
 
 // Queue one step reading buf[src_idx], writing buf[src_idx ^ 1].
 template <typename T>
-cudaError_t enqueue_step_t(tm_batch* b, int src_idx, const long long* step_base, long long step_off)
+cudaError_t enqueue_step_t(tm_batch* b, int src_idx, const long long* step_base, long long step_off, int slot)
 {
     cudaStream_t s = b->ctx->stream;
     const T* in = (const T*)b->buf[src_idx];
@@ -310,12 +310,8 @@ cudaError_t enqueue_step_t(tm_batch* b, int src_idx, const long long* step_base,
             const int grid = std::max(1, std::min(b->n_btasks, b->ctx->num_sms * 2));
             return launch_dp_det<T>(d, m.stencil, m.integrator, grid, s);
         }
-        if (b->ramped) {
-            e = launch_consts(b->d_a0, b->d_astep, b->n_inst, (4.0 * m.D) / (m.dx * m.dx), m.sigma * m.sigma, m.dt,
-                              step_base, step_off, b->d_consts, s);
-            if (e != cudaSuccess) return e;
-        }
         DornicArgs<T> a = dornic_args<T>(b, in, out, step_base, step_off);
+        if (b->ramped) a.it.consts += (long long)slot * b->n_inst;
         e = launch_dornic<T>(a, m.remainder == TM_REM_RK4 ? 1 : 0, step_grid, 256, s);
         if (e == cudaSuccess && b->spreading) e = launch_border_stop<T>(out, b->tables(), b->n_inst, s);
         return e;
@@ -333,10 +329,21 @@ cudaError_t enqueue_step_t(tm_batch* b, int src_idx, const long long* step_base,
     return launch_rk4<T>(r, false, grid_rk, s);
 }
 
-cudaError_t enqueue_step(tm_batch* b, int src_idx, const long long* step_base, long long step_off)
+// slot: the step's place in the run of steps whose constants enqueue_consts queued.
+cudaError_t enqueue_step(tm_batch* b, int src_idx, const long long* step_base, long long step_off, int slot)
 {
-    return b->precision == TM_FP64 ? enqueue_step_t<double>(b, src_idx, step_base, step_off)
-                                   : enqueue_step_t<float>(b, src_idx, step_base, step_off);
+    return b->precision == TM_FP64 ? enqueue_step_t<double>(b, src_idx, step_base, step_off, slot)
+                                   : enqueue_step_t<float>(b, src_idx, step_base, step_off, slot);
+}
+
+// Queue the Dornic constants of the next n <= kGraphSteps steps (ramped batches only: the
+// others' never change).
+cudaError_t enqueue_consts(tm_batch* b, const long long* step_base, long long step_off, int n)
+{
+    if (!b->ramped || b->model != 0 || b->dpm.deterministic) return cudaSuccess;
+    const tm_dp_model& m = b->dpm;
+    return launch_consts(b->d_a0, b->d_astep, b->n_inst, n, (4.0 * m.D) / (m.dx * m.dx), m.sigma * m.sigma, m.dt, step_base,
+                         step_off, b->d_consts, b->ctx->stream);
 }
 
 int ensure_graph(tm_batch* b, int parity)
@@ -345,8 +352,8 @@ int ensure_graph(tm_batch* b, int parity)
     cudaStream_t s = b->ctx->stream;
     cudaGraph_t g = nullptr;
     TM_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    cudaError_t e = cudaSuccess;
-    for (int k = 0; k < kGraphSteps && e == cudaSuccess; ++k) e = enqueue_step(b, (parity + k) & 1, b->d_step, k);
+    cudaError_t e = enqueue_consts(b, b->d_step, 0, kGraphSteps);
+    for (int k = 0; k < kGraphSteps && e == cudaSuccess; ++k) e = enqueue_step(b, (parity + k) & 1, b->d_step, k, k);
     cudaError_t e2 = cudaStreamEndCapture(s, &g);
     if (e != cudaSuccess || e2 != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
@@ -373,10 +380,13 @@ int run_steps(tm_batch* b, int64_t n)
             n -= kGraphSteps;
             // kGraphSteps is even: the current buffer is unchanged
         } else {
-            TM_CUDA(enqueue_step(b, b->cur, nullptr, b->step));
-            b->cur ^= 1;
-            b->step += 1;
-            n -= 1;
+            TM_CUDA(enqueue_consts(b, nullptr, b->step, (int)n));
+            for (int k = 0; k < (int)n; ++k) {
+                TM_CUDA(enqueue_step(b, b->cur, nullptr, b->step, k));
+                b->cur ^= 1;
+                b->step += 1;
+            }
+            n = 0;
         }
     }
     return TM_OK;
@@ -431,7 +441,8 @@ int batch_common_init(tm_batch* b, const tm_instance* inst, int n)
     }
     TM_CUDA(dalloc(&b->d_off, n)); TM_CUDA(dalloc(&b->d_fstride, n)); TM_CUDA(dalloc(&b->d_L, n));
     TM_CUDA(dalloc(&b->d_seed, n)); TM_CUDA(dalloc(&b->d_R, n)); TM_CUDA(dalloc(&b->d_a0, n));
-    TM_CUDA(dalloc(&b->d_astep, n)); TM_CUDA(dalloc(&b->d_consts, n)); TM_CUDA(dalloc(&b->d_alive, n));
+    TM_CUDA(dalloc(&b->d_astep, n)); TM_CUDA(dalloc(&b->d_consts, (size_t)n * (b->ramped ? kGraphSteps : 1)));
+    TM_CUDA(dalloc(&b->d_alive, n));
     TM_CUDA(dalloc(&b->d_status, n)); TM_CUDA(dalloc(&b->d_step, 1));
     TM_CUDA(cudaMemcpy(b->d_off, off.data(), n * sizeof(long long), cudaMemcpyHostToDevice));
     TM_CUDA(cudaMemcpy(b->d_fstride, fs.data(), n * sizeof(long long), cudaMemcpyHostToDevice));
@@ -585,7 +596,7 @@ int tm_batch_create_dp(tm_ctx* c, const tm_dp_model* m, const tm_instance* inst,
     for (int k = 0; k < n_inst; ++k) b->ramped = b->ramped || inst[k].a_step != 0.0;
     rc = batch_common_init(b, inst, n_inst);
     if (rc == TM_OK && !m->deterministic) {
-        if (!cuda_ok(launch_consts(b->d_a0, b->d_astep, n_inst, (4.0 * m->D) / (m->dx * m->dx),
+        if (!cuda_ok(launch_consts(b->d_a0, b->d_astep, n_inst, 1, (4.0 * m->D) / (m->dx * m->dx),
                                    m->sigma * m->sigma, m->dt, nullptr, 0, b->d_consts, c->stream)) ||
             !cuda_ok(cudaStreamSynchronize(c->stream)))
             rc = TM_ERR_CUDA;
@@ -625,7 +636,7 @@ int tm_batch_create_rietkerk(tm_ctx* c, const tm_rietkerk_model* m, const tm_ins
             (!cuda_ok(dalloc(&d_lin, n_inst)) || !cuda_ok(dalloc(&d_zero, n_inst)) ||
              !cuda_ok(cudaMemcpy(d_lin, lin.data(), n_inst * sizeof(double), cudaMemcpyHostToDevice)) ||
              !cuda_ok(cudaMemcpy(d_zero, zero.data(), n_inst * sizeof(double), cudaMemcpyHostToDevice)) ||
-             !cuda_ok(launch_consts(d_lin, d_zero, n_inst, (4.0 * m->DP) / (m->dx * m->dx), m->sigma * m->sigma,
+             !cuda_ok(launch_consts(d_lin, d_zero, n_inst, 1, (4.0 * m->DP) / (m->dx * m->dx), m->sigma * m->sigma,
                                     m->dt, nullptr, 0, b->d_consts, c->stream)) ||
              !cuda_ok(cudaStreamSynchronize(c->stream))))
             rc = TM_ERR_CUDA;

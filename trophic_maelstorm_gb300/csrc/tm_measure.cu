@@ -65,6 +65,14 @@ struct ColSum<float> {
 // spread (DP), f = 1 is the sum over occupied sites of the squared distance
 // (row - cy)^2 + (col - cx)^2 from the seed site (meansq_spread_of_vector,
 // stochasticSPDP.cpp:156-170), summed as integers; cx, cy < 0 mean L/2.
+// x > 0; FP64 by the bits (a comparison costs as much as an addition there)
+__device__ __forceinline__ bool positive(float x) { return x > 0.0f; }
+__device__ __forceinline__ bool positive(double x)
+{
+    const long long u = __double_as_longlong(x);
+    return u > 0 && u <= 0x7ff0000000000000LL;
+}
+
 constexpr int kChunk = 8;   // rows whose loads a warp issues together
 
 template <typename T>
@@ -75,6 +83,7 @@ __global__ void __launch_bounds__(256) measure_kernel(const T* state, const Inst
     const int lane = threadIdx.x & 31;
     const int gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int nw = (int)((gridDim.x * blockDim.x) >> 5);
+    pdl_wait();
     for (int t = gw; t < n_tasks; t += nw) {
         const int4 tk = tasks[t];
         const int k = tk.x;
@@ -105,8 +114,8 @@ __global__ void __launch_bounds__(256) measure_kernel(const T* state, const Inst
                 for (int j = 0; j < kChunk; ++j) {
                     if (r0 + j >= tk.w) break;
                     c0.add(v0[j]);
-                    ac += __popc(__ballot_sync(0xffffffffu, v0[j] > T(0)));
-                    if (spread && v0[j] > T(0)) {
+                    ac += __popc(__ballot_sync(0xffffffffu, positive(v0[j])));
+                    if (spread && positive(v0[j])) {
                         const long long dy = (long long)(tk.z + r0 + j) - cy, dx = (long long)x - cx;
                         sq += dy * dy + dx * dx;
                     }
@@ -135,8 +144,7 @@ cudaError_t launch_measure(const T* state, const InstTables& it, const int4* tas
                            double* partial, int grid, int block, cudaStream_t s, int spread, int cx, int cy)
 {
     if (n_tasks <= 0) return cudaSuccess;
-    measure_kernel<T><<<grid, block, 0, s>>>(state, it, tasks, n_tasks, nf, partial, spread, cx, cy);
-    return cudaGetLastError();
+    return launch_pdl(measure_kernel<T>, dim3(grid), dim3(block), 0, s, state, it, tasks, n_tasks, nf, partial, spread, cx, cy);
 }
 template cudaError_t launch_measure<float>(const float*, const InstTables&, const int4*, int, int, double*, int, int,
                                            cudaStream_t, int, int, int);
@@ -152,13 +160,17 @@ __global__ void border_stop_kernel(const T* state, const InstTables it, int n_in
 {
     const int lane = threadIdx.x & 31;
     const int k = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    pdl_wait();
     if (k >= n_inst || it.alive[k] == 0) return;
     const int L = it.L[k];
     const T* base = state + it.off[k];
     bool hit = false;
-    for (int i = lane; i < L; i += 32)
-        hit = hit || base[i] > T(0) || base[(long long)i * L] > T(0) || base[(long long)(L - 1) * L + i] > T(0) ||
-              base[(long long)i * L + L - 1] > T(0);
+    // all loads of an unrolled trip in flight together
+#pragma unroll 4
+    for (int i = lane; i < L; i += 32) {
+        const T a = base[i], b = base[(long long)i * L], c = base[(long long)(L - 1) * L + i], d = base[(long long)i * L + L - 1];
+        hit = hit | positive(a) | positive(b) | positive(c) | positive(d);
+    }
     if (__any_sync(0xffffffffu, hit) && lane == 0) it.alive[k] = 0;
 }
 
@@ -166,8 +178,7 @@ template <typename T>
 cudaError_t launch_border_stop(const T* state, const InstTables& it, int n_inst, cudaStream_t s)
 {
     if (n_inst <= 0) return cudaSuccess;
-    border_stop_kernel<T><<<(n_inst * 32 + 255) / 256, 256, 0, s>>>(state, it, n_inst);
-    return cudaGetLastError();
+    return launch_pdl(border_stop_kernel<T>, dim3((n_inst + 1) / 2), dim3(64), 0, s, state, it, n_inst);
 }
 template cudaError_t launch_border_stop<float>(const float*, const InstTables&, int, cudaStream_t);
 template cudaError_t launch_border_stop<double>(const double*, const InstTables&, int, cudaStream_t);
@@ -247,16 +258,28 @@ __global__ void finalize_kernel(const double* partial, const int* task_begin, co
 {
     const int lane = threadIdx.x & 31;
     const int k = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    pdl_wait();
     if (k >= n_inst) return;
     const int t0 = task_begin[k], t1 = task_begin[k + 1];
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0, ac = 0.0;
+    // active sites are whole numbers below 2^53, so they add as integers; sums that a
+    // measurement does not have are not formed
+    const bool has1 = nf == 3 || spread, has2 = nf == 3;
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0;
+    long long n_ac = 0;
+#pragma unroll 4
     for (int t = t0 + lane; t < t1; t += 32) {
-        s0 += partial[4LL * t + 0];
-        s1 += partial[4LL * t + 1];
-        s2 += partial[4LL * t + 2];
-        ac += partial[4LL * t + 3];
+        const double2 a = reinterpret_cast<const double2*>(partial)[2LL * t], b = reinterpret_cast<const double2*>(partial)[2LL * t + 1];
+        s0 += a.x;
+        if (has1) s1 += a.y;
+        if (has2) s2 += b.x;
+        n_ac += (long long)b.y;
     }
-    s0 = warp_sum(s0); s1 = warp_sum(s1); s2 = warp_sum(s2); ac = warp_sum(ac);
+    s0 = warp_sum(s0);
+    if (has1) s1 = warp_sum(s1);
+    if (has2) s2 = warp_sum(s2);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) n_ac += __shfl_xor_sync(0xffffffffu, n_ac, o);
+    const double ac = (double)n_ac;
     if (lane == 0) {
         const bool dead = it.alive != nullptr && it.alive[k] == 0;
         const double n = (double)it.L[k] * (double)it.L[k];
@@ -281,10 +304,8 @@ cudaError_t launch_finalize(const double* partial, const int* task_begin, const 
                             int dp_extinction, int spread, double* obs_row, cudaStream_t s)
 {
     if (n_inst <= 0) return cudaSuccess;
-    const int threads = 256;
-    const int grid = (n_inst * 32 + threads - 1) / threads;
-    finalize_kernel<<<grid, threads, 0, s>>>(partial, task_begin, it, n_inst, nf, dp_extinction, spread, obs_row);
-    return cudaGetLastError();
+    return launch_pdl(finalize_kernel, dim3((n_inst + 1) / 2), dim3(64), 0, s, partial, task_begin, it, n_inst, nf, dp_extinction,
+                      spread, obs_row);
 }
 
 }  // namespace tmg

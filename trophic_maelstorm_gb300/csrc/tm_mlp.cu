@@ -23,7 +23,7 @@
 // 53.3 us with everything unrolled (waiting for instructions), tanh evaluated twice and
 // 2-byte transposed stores; 36.4 us with loops, gelu' kept in TMEM, matrix-load
 // transposes, 16-byte constant loads, one polling warp, and both kernels' prologues overlapping
-// their predecessors (programmatic dependent launch: 43 -> 36).  512 or 1024 threads made
+// their predecessors' ends (programmatic dependent launch: 43 -> 36).  512 or 1024 threads made
 // no difference before the shared-memory work went down.
 // Every wait on an MMA completion is bounded: on timeout the CTA records an
 // error, waits once more (again bounded) for the MMAs it issued, frees its
@@ -295,7 +295,6 @@ __global__ void __launch_bounds__(NT, 1) mlp_tile_kernel(MlpArgs a)
     const uint32_t bar_a = saddr(bar);
 
     // what the update kernel does not write comes before the wait for it
-    tmg::pdl_trigger();
     float x0 = 0.0f, x1 = 0.0f, x2 = 0.0f;
     if (valid) {
         x0 = a.x[3 * s];
@@ -628,7 +627,6 @@ constexpr int kAdamGrid = (NP + kAdamParams - 1) / kAdamParams + 1;      // the 
 __global__ void __launch_bounds__(kAdamThreads) mlp_adam_kernel(AdamArgs a)
 {
     __shared__ float part[kAdamTiles][kAdamParams];
-    tmg::pdl_trigger();
     tmg::pdl_wait();
     if (a.err != nullptr && *a.err != 0) return;
     const int tid = threadIdx.x;

@@ -188,6 +188,7 @@ __global__ void __launch_bounds__(RK64_THREADS, 1) rk4_tile64_kernel(const RK4Ar
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(bar) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    pdl_wait();
     __syncthreads();
     uint32_t phase = 0;
     for (int t = blockIdx.x; t < A.n_tasks; t += gridDim.x) {
@@ -305,9 +306,7 @@ cudaError_t launch_rk4<double>(const RK4Args<double>& a, bool det, int grid, cud
         if (e != cudaSuccess) return e;
         attr[det ? 1 : 0] = true;
     }
-    if (det) rk4_tile64_kernel<true><<<grid, RK64_THREADS, smem, s>>>(a);
-    else rk4_tile64_kernel<false><<<grid, RK64_THREADS, smem, s>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(det ? rk4_tile64_kernel<true> : rk4_tile64_kernel<false>, dim3(grid), dim3(RK64_THREADS), smem, s, a);
 }
 
 // ---- noise-off DP: drho/dt = a rho - b rho^2 - c rho^3 + D Lap(rho) ---------------
@@ -348,6 +347,7 @@ __global__ void __launch_bounds__(RK_THREADS, 1) dp_det_tile_kernel(const DetTil
     T* const MA = X0 + RN;
     T* const MB = MA + RN;
     const int tid = threadIdx.x;
+    pdl_wait();
     for (int t = blockIdx.x; t < A.n_tasks; t += gridDim.x) {
         const int4 tk = A.tasks[t];
         const int k = tk.x;
@@ -436,8 +436,7 @@ cudaError_t launch_det_t(const DetTileArgs<T>& a, int grid, cudaStream_t s)
         if (e != cudaSuccess) return e;
         attr = true;
     }
-    dp_det_tile_kernel<T, RAD, NST><<<grid, RK_THREADS, smem, s>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(dp_det_tile_kernel<T, RAD, NST>, dim3(grid), dim3(RK_THREADS), smem, s, a);
 }
 
 template <typename T>

@@ -218,6 +218,7 @@ __global__ void __launch_bounds__(RK_THREADS, RK_CTAS) rk4_tile_kernel(const RK4
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(bar) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    pdl_wait();
     __syncthreads();
     uint32_t phase = 0;
     if ((int)blockIdx.x < A.n_tasks && by_copies<DET>(A, A.it.L[A.tasks[blockIdx.x].x]))
@@ -352,9 +353,7 @@ cudaError_t launch_rk4<float>(const RK4Args<float>& a, bool det, int grid, cudaS
         if (e != cudaSuccess) return e;
         attr[det ? 1 : 0] = true;
     }
-    if (det) rk4_tile_kernel<true><<<grid, RK_THREADS, smem, s>>>(a);
-    else rk4_tile_kernel<false><<<grid, RK_THREADS, smem, s>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(det ? rk4_tile_kernel<true> : rk4_tile_kernel<false>, dim3(grid), dim3(RK_THREADS), smem, s, a);
 }
 
 }  // namespace tmg

@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(256, 4) dornic_step_kernel(const DornicArgs<fl
     __shared__ SmemTab<float> tab;
     __shared__ unsigned defer_rows[kWarps][32];
     tab.fill();
+    pdl_wait();
     __syncthreads();
     const int cap = A.rows_cap * 32;
     unsigned char* wbase = smem_raw + (threadIdx.x >> 5) * warp_scratch_bytes(A.rows_cap);
@@ -274,6 +275,7 @@ __global__ void __launch_bounds__(256) dornic_deferred_kernel(const DornicArgs<f
 {
     __shared__ SmemTab<float> tab;
     tab.fill();
+    pdl_wait();
     __syncthreads();
     const long long step = (A.step_base ? *A.step_base : 0LL) + A.step_off;
     const int lane = threadIdx.x & 31;
@@ -307,9 +309,9 @@ cudaError_t launch_dornic_t(const DornicArgs<float>& a, int grid, int block, siz
     if (a.dlist == nullptr || a.dcnt == nullptr || need > a.seg_cap || (long long)n_seg > a.max_seg ||
         (long long)n_seg * a.seg_cap > a.dlist_cap)
         return cudaErrorInvalidValue;
-    dornic_step_kernel<REM, SAMP, CAP><<<grid, block, smem, s>>>(a);
-    dornic_deferred_kernel<REM, SAMP, CAP><<<(n_seg + 7) / 8, 256, 0, s>>>(a, n_seg);
-    return cudaGetLastError();
+    const cudaError_t e = launch_pdl(dornic_step_kernel<REM, SAMP, CAP>, dim3(grid), dim3(block), smem, s, a);
+    if (e != cudaSuccess) return e;
+    return launch_pdl(dornic_deferred_kernel<REM, SAMP, CAP>, dim3((n_seg + 7) / 8), dim3(256), 0, s, a, n_seg);
 }
 
 template <int REM>
@@ -337,15 +339,18 @@ cudaError_t launch_dornic<float>(const DornicArgs<float>& a, int rem, int grid, 
     return cudaErrorInvalidValue;
 }
 
-// Dornic constants per instance for the step about to run (stochasticSPDP.cpp:952-954):
-// beta = a - 4D/dx^2, lambda = 2 beta / (sigma^2 (e^{beta dt} - 1)); the beta == 0
-// limit is lambda = 2/(sigma^2 dt).  a(s) = a0 + astep * s (a ramp when astep != 0).
-__global__ void consts_kernel(const double* a0, const double* astep, int n, double diff4, double sigma2, double dt,
-                              const long long* step_base, long long step_off, Dc4* out)
+// Dornic constants of every instance for n_steps steps from the one about to run
+// (stochasticSPDP.cpp:952-954): beta = a - 4D/dx^2, lambda = 2 beta / (sigma^2 (e^{beta dt}
+// - 1)); the beta == 0 limit is lambda = 2/(sigma^2 dt).  a(s) = a0 + astep * s (a ramp when
+// astep != 0).  out[j n + k]: step j, instance k -- one launch for a run of steps.
+__global__ void consts_kernel(const double* a0, const double* astep, int n, int n_steps, double diff4, double sigma2,
+                              double dt, const long long* step_base, long long step_off, Dc4* out)
 {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const long long step = (step_base ? *step_base : 0LL) + step_off;
+    pdl_wait();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n * n_steps) return;
+    const int j = i / n, k = i - j * n;
+    const long long step = (step_base ? *step_base : 0LL) + step_off + j;
     const double a = a0[k] + astep[k] * (double)step;
     const double beta = a - diff4;
     const double e = tm_exp(beta * dt);
@@ -357,15 +362,15 @@ __global__ void consts_kernel(const double* a0, const double* astep, int n, doub
         lambda = (2.0 * beta) / (sigma2 * (e - 1.0));
         m2 = (e - 1.0) / beta;
     }
-    out[k] = Dc4{lambda * e, 1.0 / lambda, e, m2};
+    out[i] = Dc4{lambda * e, 1.0 / lambda, e, m2};
 }
 
-cudaError_t launch_consts(const double* a0, const double* astep, int n, double diff4, double sigma2, double dt,
+cudaError_t launch_consts(const double* a0, const double* astep, int n, int n_steps, double diff4, double sigma2, double dt,
                           const long long* step_base, long long step_off, Dc4* out, cudaStream_t s)
 {
-    if (n <= 0) return cudaSuccess;
-    consts_kernel<<<(n + 127) / 128, 128, 0, s>>>(a0, astep, n, diff4, sigma2, dt, step_base, step_off, out);
-    return cudaGetLastError();
+    if (n <= 0 || n_steps <= 0) return cudaSuccess;
+    return launch_pdl(consts_kernel, dim3((unsigned)(((long long)n * n_steps + 127) / 128)), dim3(128), 0, s, a0, astep, n,
+                      n_steps, diff4, sigma2, dt, step_base, step_off, out);
 }
 
 __global__ void set_step_kernel(long long* d, long long v) { *d = v; }

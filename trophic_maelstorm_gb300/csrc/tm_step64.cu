@@ -338,6 +338,7 @@ __global__ void __launch_bounds__(256, 2) dornic_step64_kernel(const DornicArgs<
     __shared__ Tab64 tab;
     __shared__ int left[kWarps][3];
     tab.fill_all();
+    pdl_wait();
     __syncthreads();
     const int warp = threadIdx.x >> 5;
     unsigned char* const wbase = smem_raw + warp * warp_bytes(A.rows_cap);
@@ -572,8 +573,7 @@ cudaError_t launch64_t(const DornicArgs<double>& a, int grid, int block, cudaStr
         if (e != cudaSuccess) return e;
         attr_set = true;
     }
-    dornic_step64_kernel<REM, SAMP, CAP><<<grid, block, warp_bytes(a.rows_cap) * kWarps, s>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(dornic_step64_kernel<REM, SAMP, CAP>, dim3(grid), dim3(block), warp_bytes(a.rows_cap) * kWarps, s, a);
 }
 
 template <int REM>
