@@ -100,6 +100,7 @@ struct tm_batch {
     int obs_cap = 0;
 
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
+    SpectrumWork* spectrum = nullptr;   // of the last power spectrum's side and bin width
 
     InstTables tables() const
     {
@@ -558,6 +559,7 @@ int tm_batch_destroy(tm_batch* b)
     cudaSetDevice(b->ctx->device);
     cudaStreamSynchronize(b->ctx->stream);
     free_graphs(b);
+    spectrum_work_destroy(b->spectrum);
     cudaFree(b->buf[0]); cudaFree(b->buf[1]); cudaFree(b->aux); cudaFree(b->site_b);
     cudaFree(b->d_dlist); cudaFree(b->d_dcnt);
     cudaFree(b->d_step); cudaFree(b->d_off); cudaFree(b->d_fstride); cudaFree(b->d_L); cudaFree(b->d_seed);
@@ -963,15 +965,15 @@ int tm_batch_power_spectrum(tm_batch* b, int k, int field, double binwidth, doub
     if (b->model == 0) TM_CUDA(cudaMemcpy(&alive, b->d_alive + k, sizeof(int), cudaMemcpyDeviceToHost));
     if (!alive) {  // an extinct instance is all zeros: no power at any k
         const int L = b->inst[k].L;
-        int rc = tm_power_spectrum_device(b->buf[b->cur], b->precision, L, binwidth, b->ctx->stream, kvals, power,
-                                          max_bins, n_bins);
+        int rc = power_spectrum(b->buf[b->cur], b->precision, L, binwidth, b->ctx->stream, kvals, power, max_bins, n_bins,
+                                &b->spectrum);
         if (rc == TM_OK)
             for (int i = 0; i < *n_bins; ++i) power[i] = 0.0;
         return rc;
     }
     const char* base = (const char*)b->buf[b->cur] + (size_t)(b->off[k] + field * b->fstride[k]) * b->esize;
-    return tm_power_spectrum_device(base, b->precision, b->inst[k].L, binwidth, b->ctx->stream, kvals, power,
-                                    max_bins, n_bins);
+    return power_spectrum(base, b->precision, b->inst[k].L, binwidth, b->ctx->stream, kvals, power, max_bins, n_bins,
+                          &b->spectrum);
 }
 
 static int run_common(tm_batch* b, const void* init, int64_t n_steps, const int64_t* meas, int n_meas, double* obs,

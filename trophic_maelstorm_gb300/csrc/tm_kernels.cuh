@@ -12,6 +12,12 @@ struct tm_ctx {
     unsigned probe = 0;            // TM_PROBE_* flags for objects created from now on (tests)
 };
 
+// tm_spectrum.cu: plan and buffers of a power spectrum, kept by their batch
+struct SpectrumWork;
+void spectrum_work_destroy(SpectrumWork* w);
+int power_spectrum(const void* dev_field, int precision, int L, double binwidth, cudaStream_t s, double* kvals,
+                   double* power, int max_bins, int* n_bins, SpectrumWork** keep);
+
 namespace tmg {
 
 // Programmatic dependent launch: a kernel launched by launch_pdl may start while the last

@@ -9,15 +9,20 @@
 // turns them into NaN afterwards).  The wavelength is L / k at the peak.
 //
 // The FFT is cuFFT's D2Z (half spectrum); columns with a mirror image count
-// twice.  The bins depend only on L, so the elements of each bin are listed
-// once on the host (CSR) and each bin is summed by one warp in list order:
-// the result does not depend on scheduling.
+// twice.  k^2 is a whole number, so each annulus is a range of whole numbers
+// [T_b, T_b+1) found once on the host, and a block sums one annulus straight from the
+// spectrum: a row's columns in it are one interval.  (Listing every element of every
+// annulus on the host took most of a call's time.)  Rows go to threads in order and
+// their sums combine in a fixed tree: the result does not depend on scheduling.
+// Plans and buffers live in a SpectrumWork, which a batch keeps for its next call.
+#include "tm_f64.cuh"
 #include "tm_kernels.cuh"
 #include "../../include/tm.h"
 
 #include <cuda_runtime.h>
 #include <cufft.h>
 #include <cmath>
+#include <new>
 #include <vector>
 
 namespace {
@@ -62,41 +67,73 @@ __global__ void normalise_kernel(const T* f, long long n, const double* mx, doub
 {
     const double m = *mx;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        out[i] = (double)f[i] / m;
+        out[i] = tmf::div((double)f[i], m);
 }
 
-// one warp per bin: sum of w * |F|^2 over the bin's listed elements, in list order
-__global__ void bin_kernel(const cufftDoubleComplex* F, const int* ptr, const int* idx, const unsigned char* w,
-                           int nbins, const double* area, double* power)
+// largest x >= 0 with x x <= n, for 0 <= n < 2^33
+__device__ __forceinline__ int isqrt(long long n)
 {
-    const int lane = threadIdx.x & 31;
-    const int b = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    if (b >= nbins) return;
-    double s = 0.0, c = 0.0;
-    for (int j = ptr[b] + lane; j < ptr[b + 1]; j += 32) {
-        const cufftDoubleComplex z = F[idx[j]];
-        const double p = z.x * z.x + z.y * z.y;
-        s += (double)w[j] * p;
-        c += (double)w[j];
+    int r = (int)sqrtf((float)n);
+    while ((long long)r * r > n) --r;
+    while ((long long)(r + 1) * (r + 1) <= n) ++r;
+    return r;
+}
+
+constexpr int kBinThreads = 128;
+
+// one block per annulus: mean of |F|^2 over the modes with lim[b] <= k^2 < lim[b + 1],
+// times its area
+__global__ void __launch_bounds__(kBinThreads) bin_kernel(const cufftDoubleComplex* F, int L, const long long* lim,
+                                                          const double* area, double* power)
+{
+    __shared__ double red[kBinThreads / 32];
+    __shared__ unsigned long long cred[kBinThreads / 32];
+    const int b = blockIdx.x, nx = L / 2 + 1;
+    const long long lo = lim[b], hi = lim[b + 1] - 1;         // k^2 in [lo, hi]
+    const int fmax = (L - 1) / 2, fmin = -(L / 2);              // row frequencies
+    const int R = hi < 0 ? -1 : isqrt(hi);
+    double s = 0.0;
+    unsigned long long c = 0;
+    for (int fy = max(fmin, -R) + (int)threadIdx.x; fy <= min(fmax, R); fy += kBinThreads) {
+        const long long f2 = (long long)fy * fy;
+        const int x1 = min(nx - 1, isqrt(hi - f2));
+        const int x0 = lo - f2 <= 0 ? 0 : isqrt(lo - f2 - 1) + 1;
+        const cufftDoubleComplex* row = F + (long long)(fy < 0 ? fy + L : fy) * nx;
+        for (int x = x0; x <= x1; ++x) {
+            const cufftDoubleComplex z = row[x];
+            const double p = fma(z.x, z.x, z.y * z.y);
+            const bool twice = x >= 1 && x <= (L - 1) / 2;     // the mirror column's mode
+            s = twice ? fma(2.0, p, s) : s + p;
+            c += twice ? 2 : 1;
+        }
     }
     s = wsum(s);
-    c = wsum(c);
-    if (lane == 0) power[b] = (c != 0.0) ? (s / c) * area[b] : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    if ((threadIdx.x & 31) == 0) {
+        red[threadIdx.x >> 5] = s;
+        cred[threadIdx.x >> 5] = c;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kBinThreads / 32; ++w) {
+            s += red[w];
+            c += cred[w];
+        }
+        power[b] = c ? (s / (double)c) * area[b] : 0.0;
+    }
 }
 
-struct Plan {
-    int L = 0;
-    double bw = 0;
+// Annuli of a lattice: centres, areas, and the limits of k^2: lim[b] is the least whole
+// n with sqrt(n) >= e_b, the last one the least with sqrt(n) > e_nbins (that bin is closed).
+struct Annuli {
     int nbins = 0;
     std::vector<double> kvals, area;
-    std::vector<int> ptr, idx;
-    std::vector<unsigned char> w;
+    std::vector<long long> lim;
 };
 
-void make_plan(int L, double bw, Plan& p)
+void make_annuli(int L, double bw, Annuli& p)
 {
-    p.L = L;
-    p.bw = bw;
     // edges: numpy.arange(1 - bw/2, L//2 + 1, bw)
     std::vector<double> e;
     const double start = 1.0 - bw / 2.0, stop = (double)(L / 2 + 1);
@@ -109,93 +146,129 @@ void make_plan(int L, double bw, Plan& p)
         p.kvals[b] = 0.5 * (e[b + 1] + e[b]);
         p.area[b] = M_PI * (e[b + 1] * e[b + 1] - e[b] * e[b]);
     }
-    const int nx = L / 2 + 1;
-    std::vector<std::vector<int>> per(p.nbins);
-    std::vector<std::vector<unsigned char>> pw(p.nbins);
-    for (int ky = 0; ky < L; ++ky) {
-        const long long fy = (ky <= (L - 1) / 2) ? ky : ky - L;
-        for (int kx = 0; kx < nx; ++kx) {
-            const double k = std::sqrt((double)(kx * (long long)kx + fy * fy));
-            if (p.nbins == 0 || k < e[0] || k > e[p.nbins]) continue;
-            int b = (int)((k - e[0]) / bw);
-            if (b >= p.nbins) b = p.nbins - 1;
-            while (b > 0 && k < e[b]) --b;
-            while (b < p.nbins - 1 && k >= e[b + 1]) ++b;
-            const bool mirrored = kx >= 1 && kx <= (L - 1) / 2;
-            per[b].push_back(ky * nx + kx);
-            pw[b].push_back(mirrored ? 2 : 1);
-        }
-    }
-    p.ptr.assign(p.nbins + 1, 0);
-    for (int b = 0; b < p.nbins; ++b) p.ptr[b + 1] = p.ptr[b] + (int)per[b].size();
-    p.idx.clear();
-    p.w.clear();
-    for (int b = 0; b < p.nbins; ++b) {
-        p.idx.insert(p.idx.end(), per[b].begin(), per[b].end());
-        p.w.insert(p.w.end(), pw[b].begin(), pw[b].end());
+    p.lim.clear();
+    for (size_t i = 0; i < e.size() && p.nbins; ++i) {
+        if (e[i] <= 0.0) { p.lim.push_back(0); continue; }
+        const bool last = i + 1 == e.size();
+        auto below = [&](long long n) { return last ? std::sqrt((double)n) <= e[i] : std::sqrt((double)n) < e[i]; };
+        long long n = (long long)(e[i] * e[i]);
+        while (n > 0 && !below(n - 1)) --n;
+        while (below(n)) ++n;
+        p.lim.push_back(n);
     }
 }
 
+#define SPEC_CUDA(call)                                        \
+    do {                                                       \
+        if ((call) != cudaSuccess) {                           \
+            (void)cudaGetLastError();                          \
+            return TM_ERR_CUDA;                                \
+        }                                                      \
+    } while (0)
+
 }  // namespace
+
+// Device buffers and FFT plan for one lattice side and bin width.
+struct SpectrumWork {
+    int L = 0;
+    double bw = 0.0;
+    Annuli ann;
+    bool have_plan = false;
+    cufftHandle plan = 0;
+    double *img = nullptr, *part = nullptr, *area = nullptr, *power = nullptr;
+    long long* lim = nullptr;
+    cufftDoubleComplex* F = nullptr;
+    static constexpr int kBlocks = 304;
+
+    ~SpectrumWork()
+    {
+        if (have_plan) cufftDestroy(plan);
+        for (void* q : {(void*)img, (void*)part, (void*)area, (void*)power, (void*)lim, (void*)F}) cudaFree(q);
+        (void)cudaGetLastError();
+    }
+
+    // Plan and buffers (nothing of them when the lattice has no annulus).
+    int prepare(cudaStream_t s)
+    {
+        if (ann.nbins == 0) return TM_OK;
+        const size_t n = (size_t)L * L;
+        SPEC_CUDA(cudaMalloc(&img, n * sizeof(double)));
+        SPEC_CUDA(cudaMalloc(&F, (size_t)L * (L / 2 + 1) * sizeof(cufftDoubleComplex)));
+        SPEC_CUDA(cudaMalloc(&part, kBlocks * sizeof(double)));
+        SPEC_CUDA(cudaMalloc(&area, ann.nbins * sizeof(double)));
+        SPEC_CUDA(cudaMalloc(&power, ann.nbins * sizeof(double)));
+        SPEC_CUDA(cudaMalloc(&lim, ann.lim.size() * sizeof(long long)));
+        SPEC_CUDA(cudaMemcpyAsync(area, ann.area.data(), ann.nbins * sizeof(double), cudaMemcpyHostToDevice, s));
+        SPEC_CUDA(cudaMemcpyAsync(lim, ann.lim.data(), ann.lim.size() * sizeof(long long), cudaMemcpyHostToDevice, s));
+        if (cufftPlan2d(&plan, L, L, CUFFT_D2Z) != CUFFT_SUCCESS) return TM_ERR_CUDA;
+        have_plan = true;
+        return cufftSetStream(plan, s) == CUFFT_SUCCESS ? TM_OK : TM_ERR_CUDA;
+    }
+
+    template <typename T>
+    int run(const T* field, cudaStream_t s, double* kvals, double* out)
+    {
+        const long long n = (long long)L * L;
+        max_partial_kernel<T><<<kBlocks, 256, 0, s>>>(field, n, part);
+        max_final_kernel<<<1, 32, 0, s>>>(part, kBlocks);
+        normalise_kernel<T><<<kBlocks, 256, 0, s>>>(field, n, part, img);
+        SPEC_CUDA(cudaGetLastError());
+        if (cufftExecD2Z(plan, img, F) != CUFFT_SUCCESS) return TM_ERR_CUDA;
+        bin_kernel<<<ann.nbins, kBinThreads, 0, s>>>(F, L, lim, area, power);
+        SPEC_CUDA(cudaGetLastError());
+        SPEC_CUDA(cudaMemcpyAsync(out, power, ann.nbins * sizeof(double), cudaMemcpyDeviceToHost, s));
+        SPEC_CUDA(cudaStreamSynchronize(s));
+        for (int b = 0; b < ann.nbins; ++b) kvals[b] = ann.kvals[b];
+        return TM_OK;
+    }
+};
+
+void spectrum_work_destroy(SpectrumWork* w) { delete w; }
+
+// Spectrum of a device field; *keep (may be null) is a SpectrumWork of an earlier call, used
+// when side and bin width are the same and replaced otherwise.  One host thread and one
+// stream at a time, as its owner's.
+int power_spectrum(const void* dev_field, int precision, int L, double binwidth, cudaStream_t s, double* kvals,
+                   double* power, int max_bins, int* n_bins, SpectrumWork** keep)
+{
+    if (!dev_field || L < 2 || !(binwidth > 0) || !kvals || !power || !n_bins || max_bins < 0) return TM_ERR_INVALID;
+    if (precision != TM_FP64 && precision != TM_FP32) return TM_ERR_INVALID;
+    SpectrumWork* w = keep ? *keep : nullptr;
+    if (!w || w->L != L || w->bw != binwidth) {
+        SpectrumWork* fresh = new (std::nothrow) SpectrumWork;
+        if (!fresh) return TM_ERR_NOMEM;
+        fresh->L = L;
+        fresh->bw = binwidth;
+        make_annuli(L, binwidth, fresh->ann);
+        *n_bins = fresh->ann.nbins;
+        if (fresh->ann.nbins > max_bins || fresh->ann.nbins == 0) {
+            const int rc = fresh->ann.nbins > max_bins ? TM_ERR_INVALID : TM_OK;
+            delete fresh;
+            return rc;
+        }
+        if (keep) {
+            delete w;                       // first, so that both never hold memory together
+            *keep = nullptr;
+        }
+        const int rc = fresh->prepare(s);
+        if (rc != TM_OK) {
+            delete fresh;
+            return rc;
+        }
+        w = fresh;
+        if (keep) *keep = w;
+    }
+    *n_bins = w->ann.nbins;
+    int rc = TM_ERR_INVALID;
+    if (w->ann.nbins <= max_bins)
+        rc = precision == TM_FP64 ? w->run((const double*)dev_field, s, kvals, power)
+                                  : w->run((const float*)dev_field, s, kvals, power);
+    if (!keep) delete w;
+    return rc;
+}
 
 extern "C" int tm_power_spectrum_device(const void* dev_field, int precision, int L, double binwidth, void* stream,
                                         double* kvals, double* power, int max_bins, int* n_bins)
 {
-    if (!dev_field || L < 2 || !(binwidth > 0) || !kvals || !power || !n_bins || max_bins < 0) return TM_ERR_INVALID;
-    if (precision != TM_FP64 && precision != TM_FP32) return TM_ERR_INVALID;
-    Plan p;
-    make_plan(L, binwidth, p);
-    *n_bins = p.nbins;
-    if (p.nbins > max_bins) return TM_ERR_INVALID;
-    if (p.nbins == 0) return TM_OK;
-    cudaStream_t s = (cudaStream_t)stream;
-    const long long n = (long long)L * L;
-    const int nx = L / 2 + 1;
-    double* img = nullptr;
-    cufftDoubleComplex* F = nullptr;
-    double *part = nullptr, *d_area = nullptr, *d_pow = nullptr;
-    int *d_ptr = nullptr, *d_idx = nullptr;
-    unsigned char* d_w = nullptr;
-    int rc = TM_OK;
-    cufftHandle plan = 0;
-    bool have_plan = false;
-    const int nblk = 304;
-    auto ok = [&](cudaError_t e) { if (e != cudaSuccess && rc == TM_OK) rc = TM_ERR_CUDA; return rc == TM_OK; };
-    if (ok(cudaMalloc(&img, n * sizeof(double))) && ok(cudaMalloc(&F, (size_t)L * nx * sizeof(cufftDoubleComplex))) &&
-        ok(cudaMalloc(&part, nblk * sizeof(double))) && ok(cudaMalloc(&d_area, p.nbins * sizeof(double))) &&
-        ok(cudaMalloc(&d_pow, p.nbins * sizeof(double))) && ok(cudaMalloc(&d_ptr, (p.nbins + 1) * sizeof(int))) &&
-        ok(cudaMalloc(&d_idx, p.idx.size() * sizeof(int) + 4)) && ok(cudaMalloc(&d_w, p.w.size() + 4)) &&
-        ok(cudaMemcpyAsync(d_area, p.area.data(), p.nbins * sizeof(double), cudaMemcpyHostToDevice, s)) &&
-        ok(cudaMemcpyAsync(d_ptr, p.ptr.data(), (p.nbins + 1) * sizeof(int), cudaMemcpyHostToDevice, s)) &&
-        ok(cudaMemcpyAsync(d_idx, p.idx.data(), p.idx.size() * sizeof(int), cudaMemcpyHostToDevice, s)) &&
-        ok(cudaMemcpyAsync(d_w, p.w.data(), p.w.size(), cudaMemcpyHostToDevice, s))) {
-        if (precision == TM_FP64) {
-            max_partial_kernel<double><<<nblk, 256, 0, s>>>((const double*)dev_field, n, part);
-            max_final_kernel<<<1, 32, 0, s>>>(part, nblk);
-            normalise_kernel<double><<<nblk, 256, 0, s>>>((const double*)dev_field, n, part, img);
-        } else {
-            max_partial_kernel<float><<<nblk, 256, 0, s>>>((const float*)dev_field, n, part);
-            max_final_kernel<<<1, 32, 0, s>>>(part, nblk);
-            normalise_kernel<float><<<nblk, 256, 0, s>>>((const float*)dev_field, n, part, img);
-        }
-        ok(cudaGetLastError());
-        if (rc == TM_OK && cufftPlan2d(&plan, L, L, CUFFT_D2Z) == CUFFT_SUCCESS) {
-            have_plan = true;
-            if (cufftSetStream(plan, s) != CUFFT_SUCCESS || cufftExecD2Z(plan, img, F) != CUFFT_SUCCESS) rc = TM_ERR_CUDA;
-        } else if (rc == TM_OK) {
-            rc = TM_ERR_CUDA;
-        }
-        if (rc == TM_OK) {
-            bin_kernel<<<(p.nbins * 32 + 255) / 256, 256, 0, s>>>(F, d_ptr, d_idx, d_w, p.nbins, d_area, d_pow);
-            ok(cudaGetLastError());
-            ok(cudaMemcpyAsync(power, d_pow, p.nbins * sizeof(double), cudaMemcpyDeviceToHost, s));
-            ok(cudaStreamSynchronize(s));
-            for (int b = 0; b < p.nbins; ++b) kvals[b] = p.kvals[b];
-        }
-    }
-    if (have_plan) cufftDestroy(plan);
-    cudaFree(img); cudaFree(F); cudaFree(part); cudaFree(d_area); cudaFree(d_pow);
-    cudaFree(d_ptr); cudaFree(d_idx); cudaFree(d_w);
-    (void)cudaGetLastError();
-    return rc;
+    return power_spectrum(dev_field, precision, L, binwidth, (cudaStream_t)stream, kvals, power, max_bins, n_bins, nullptr);
 }
