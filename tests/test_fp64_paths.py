@@ -144,3 +144,28 @@ def test_fp64_draw_paths_match_oracle(oracle, dt, scale, sampler, remainder):
         _, _, want, ost = oracle.dp_run(p, init[k], 5 + k, 7, [7])
         assert np.array_equal(fin[k], want), (k, L)
         assert st[k] == ost
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sampler", [0, 1])
+@pytest.mark.parametrize("dt", [0.02, 0.004, 0.0007], ids=["m100", "m500", "m2900"])
+def test_fp64_transformed_rejection_matches_oracle(oracle, dt, sampler):
+    """Poisson means through 32, 100 and 4096 (where the FP32 decisions end), bit for bit."""
+    import trophic_maelstorm_gb300 as tmg
+    ctx = tmg.Context(0)
+    rng = np.random.default_rng(11)
+    Ls = [33, 130]
+    model = tmg.dp_model(dt=dt, sampler=sampler)
+    b = tmg.Batch(ctx, model, tmg.instances(Ls, [3, 4], 0.53), tmg.TM_FP64)
+    init = [rng.uniform(0.0, 3.0, (L, L)) ** 2 for L in Ls]
+    b.upload(init)
+    _, st = b.advance(5, [])
+    fin = b.download()
+    b.close()
+    ctx.close()
+    for k, L in enumerate(Ls):
+        p = oracle.DPParams(0.53, 0.0, model.b, model.c, model.D, model.sigma, model.dt, model.dx, model.clamp_lo,
+                            model.clamp_eps, model.remainder, model.sampler)
+        _, _, want, ost = oracle.dp_run(p, init[k], 3 + k, 5, [5])
+        assert np.array_equal(fin[k], want), (k, L)
+        assert st[k] == ost
