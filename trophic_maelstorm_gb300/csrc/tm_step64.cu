@@ -421,17 +421,18 @@ __global__ void __launch_bounds__(256, 2) dornic_step64_kernel(const DornicArgs<
     const long long step = (A.step_base ? *A.step_base : 0LL) + A.step_off;
     int cnt[3] = {0, 0, 0};
     // one more trip after the last task empties the lists of the whole block together
+    int4 next = A.tasks[gw < A.n_tasks ? gw : 0];
     for (int t = gw;; t += nw) {
         const bool more = t < A.n_tasks;
-        int k = 0, L = 0, x0 = 0, y0 = 0, nq = 0;
-        if (more) k = A.tasks[t].x;
-        if (more && (A.it.alive == nullptr || A.it.alive[k] != 0)) {
-            const int4 tk = A.tasks[t];
-            L = A.it.L[k];
-            const double* __restrict__ src = A.in + A.it.off[k];
-            x0 = tk.y;
-            y0 = tk.z;
-            const int rows = tk.w;
+        // the next task is asked for a trip ahead, its instance's tables in one round
+        const int4 tk = next;
+        const int k = tk.x, x0 = tk.y, y0 = tk.z, rows = tk.w;
+        const int L = A.it.L[k], alive = A.it.alive ? A.it.alive[k] : 1;
+        const long long off = A.it.off[k];
+        if (t + nw < A.n_tasks) next = A.tasks[t + nw];
+        int nq = 0;
+        if (more && alive != 0) {
+            const double* __restrict__ src = A.in + off;
             const int w = min(32, L - x0);
             const int x = x0 + lane;
             const bool act = lane < w;
@@ -440,23 +441,32 @@ __global__ void __launch_bounds__(256, 2) dornic_step64_kernel(const DornicArgs<
             const bool erow = lane < rows;
             const int xw = (x0 == 0) ? L - 1 : x0 - 1;
             const int xe = (x0 + w == L) ? 0 : x0 + w;
-            const unsigned wm =
-                __ballot_sync(0xffffffffu, erow && !tmf::is_zero(erow ? src[(long long)(y0 + lane) * L + xw] : 0.0));
-            const unsigned em =
-                __ballot_sync(0xffffffffu, erow && !tmf::is_zero(erow ? src[(long long)(y0 + lane) * L + xe] : 0.0));
             const int yn = (y0 == 0) ? L - 1 : y0 - 1;
-            const unsigned actm = __ballot_sync(0xffffffffu, act);
-            unsigned mn = __ballot_sync(0xffffffffu, act && !tmf::is_zero(act ? src[(long long)yn * L + x] : 0.0));
-            unsigned mc = __ballot_sync(0xffffffffu, act && !tmf::is_zero(act ? src[(long long)y0 * L + x] : 0.0));
-            unsigned st = 0;
-            for (int r0 = 0; r0 < rows; r0 += 8) {
-                double v[8];
+            // Every load of the pass is issued before the first vote waits for one: each vote
+            // in between cost a round trip to the L2, and an empty task 4.6k cycles instead
+            // of 2.7k (64 spreading lattices of 101^2, 200 steps: 6.20 -> 5.19 ms).
+            const double vw = erow ? src[(long long)(y0 + lane) * L + xw] : 0.0;
+            const double ve = erow ? src[(long long)(y0 + lane) * L + xe] : 0.0;
+            const double vn = act ? src[(long long)yn * L + x] : 0.0;
+            const double vc = act ? src[(long long)y0 * L + x] : 0.0;
+            double v[8];
+            const auto load8 = [&](int r0) {
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
                     int y = y0 + r0 + j + 1;
                     if (y >= L) y -= L;
                     v[j] = (act && r0 + j < rows) ? src[(long long)y * L + x] : 0.0;
                 }
+            };
+            load8(0);
+            const unsigned wm = __ballot_sync(0xffffffffu, !tmf::is_zero(vw));
+            const unsigned em = __ballot_sync(0xffffffffu, !tmf::is_zero(ve));
+            const unsigned actm = __ballot_sync(0xffffffffu, act);
+            unsigned mn = __ballot_sync(0xffffffffu, !tmf::is_zero(vn));
+            unsigned mc = __ballot_sync(0xffffffffu, !tmf::is_zero(vc));
+            unsigned st = 0;
+            for (int r0 = 0; r0 < rows; r0 += 8) {
+                if (r0 > 0) load8(r0);
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
                     const int r = r0 + j;
@@ -468,7 +478,7 @@ __global__ void __launch_bounds__(256, 2) dornic_step64_kernel(const DornicArgs<
                     if ((lm >> lane) & 1u) {
                         Wq[nq + __popc(lm & lt_mask)] = (unsigned short)(r * 32 + lane);
                     } else if (act) {
-                        const long long o = A.it.off[k] + (long long)(y0 + r) * L + x;
+                        const long long o = off + (long long)(y0 + r) * L + x;
                         double res = 0.0;
                         if (!A.zero_fixed) res = finish64<REM>(A, 0.0, A.site_b ? A.site_b[o] : A.b, st);
                         A.out[o] = res;
@@ -496,7 +506,7 @@ __global__ void __launch_bounds__(256, 2) dornic_step64_kernel(const DornicArgs<
                 const int y = y0 + (li >> 5), x = x0 + (li & 31);
                 const uint32_t site = (uint32_t)y * (uint32_t)L + (uint32_t)x;
                 en.site = site;
-                const SiteMean s = site_mean(A, A.in + A.it.off[k], L, y, x, cs.x);
+                const SiteMean s = site_mean(A, A.in + off, L, y, x, cs.x);
                 double rs = 0.0;               // also where the neighbours cancel or their sum underflows
                 if (SAMP == 2) {
                     rs = cs.z * s.cur + cs.w * s.alpha;
