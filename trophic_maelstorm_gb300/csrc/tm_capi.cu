@@ -96,6 +96,7 @@ struct tm_batch {
     int4* d_btasks = nullptr;
     int n_btasks = 0;
     double* d_partial = nullptr;
+    int n_groups = 0;                   // of a measurement's sums
     double* d_obs = nullptr;
     int obs_cap = 0;
 
@@ -187,7 +188,11 @@ int build_tasks(tm_batch* b)
     cudaFree(b->d_partial); b->d_partial = nullptr;
     b->n_tasks = (int)tasks.size();
     TM_CUDA(dalloc(&b->d_tasks, tasks.size()));
-    TM_CUDA(dalloc(&b->d_partial, 4 * tasks.size()));
+    // partials and group sums (four numbers each), then the arrival counters
+    b->n_groups = measure_group_base(b->n_tasks, b->n_inst) + 1;
+    const size_t rows = 4 * (tasks.size() + b->n_groups), counters = (size_t)b->n_inst + b->n_groups;
+    TM_CUDA(dalloc(&b->d_partial, rows + (counters + 1) / 2));
+    TM_CUDA(cudaMemset(b->d_partial + rows, 0, counters * sizeof(int)));
     TM_CUDA(cudaMemcpy(b->d_tasks, tasks.data(), tasks.size() * sizeof(int4), cudaMemcpyHostToDevice));
     if (!b->d_task_begin) TM_CUDA(dalloc(&b->d_task_begin, begin.size()));
     TM_CUDA(cudaMemcpy(b->d_task_begin, begin.data(), begin.size() * sizeof(int), cudaMemcpyHostToDevice));
@@ -393,25 +398,26 @@ int run_steps(tm_batch* b, int64_t n)
     return TM_OK;
 }
 
-int measure_into(tm_batch* b, int j)
+template <typename T>
+int measure_as(tm_batch* b, int j)
 {
-    cudaStream_t s = b->ctx->stream;
-    const int W = obs_w(b);
-    InstTables it = b->tables();
-    if (b->model == 1) it.alive = nullptr;
-    const int grid = warp_grid(b, b->n_tasks);
-    cudaError_t e;
-    if (b->precision == TM_FP64)
-        e = launch_measure<double>((const double*)b->buf[b->cur], it, b->d_tasks, b->n_tasks, b->nf, b->d_partial,
-                                   grid, 256, s, b->spreading, b->spread_cx, b->spread_cy);
-    else
-        e = launch_measure<float>((const float*)b->buf[b->cur], it, b->d_tasks, b->n_tasks, b->nf, b->d_partial, grid,
-                                  256, s, b->spreading, b->spread_cx, b->spread_cy);
-    TM_CUDA(e);
-    TM_CUDA(launch_finalize(b->d_partial, b->d_task_begin, it, b->n_inst, b->nf, b->model == 0, b->spreading,
-                            b->d_obs + (size_t)j * b->n_inst * W, s));
+    MeasureArgs<T> a{};
+    a.state = (const T*)b->buf[b->cur];
+    a.it = b->tables();
+    if (b->model == 1) a.it.alive = nullptr;
+    a.tasks = b->d_tasks; a.begin = b->d_task_begin;
+    a.n_tasks = b->n_tasks; a.n_inst = b->n_inst; a.nf = b->nf;
+    a.spread = b->spreading; a.scx = b->spread_cx; a.scy = b->spread_cy;
+    a.dp_extinction = b->model == 0;
+    a.partial = b->d_partial;
+    a.group_sums = b->d_partial + 4LL * b->n_tasks;
+    a.arrived = (int*)(a.group_sums + 4LL * b->n_groups);
+    a.obs_row = b->d_obs + (size_t)j * b->n_inst * obs_w(b);
+    TM_CUDA(launch_measure<T>(a, warp_grid(b, b->n_tasks), 256, b->ctx->stream));
     return TM_OK;
 }
+
+int measure_into(tm_batch* b, int j) { return b->precision == TM_FP64 ? measure_as<double>(b, j) : measure_as<float>(b, j); }
 
 int validate_instances(const tm_instance* inst, int n)
 {

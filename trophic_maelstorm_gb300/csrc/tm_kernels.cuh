@@ -101,6 +101,36 @@ struct RK4Args {
     int probe_no_copy;             // TM_PROBE_TILE_WAIT: issue no copy, so the bounded wait runs out
 };
 
+// Measurements.  partial[t*4 + f] of task t: f = 0..nf-1 field sums, 3 = sites with field
+// 0 > 0.  With spread (DP), f = 1 is the sum over occupied sites of the squared distance
+// (row - cy)^2 + (col - cx)^2 from the seed site (meansq_spread_of_vector,
+// stochasticSPDP.cpp:156-170), summed as integers; scx, scy < 0 mean L/2.
+constexpr int kMeasureOnce = 512;      // an instance with more tasks is summed in groups
+constexpr int kMeasureGroupShift = 8;  // groups of 256 tasks at least
+__host__ __device__ inline int measure_group_shift(int nt)
+{
+    int sh = kMeasureGroupShift;
+    while ((1LL << (2 * sh)) < nt) ++sh;
+    return sh;
+}
+// First group of instance k, whose tasks start at b0: up to floor(n / 256) + 1 groups of
+// its n tasks end before the next instance's first.
+__host__ __device__ inline int measure_group_base(int b0, int k) { return (b0 >> kMeasureGroupShift) + k; }
+template <typename T>
+struct MeasureArgs {
+    const T* state;
+    InstTables it;
+    const int4* tasks;
+    const int* begin;              // first task of each instance, and n_tasks
+    int n_tasks, n_inst, nf;
+    int spread, scx, scy;
+    int dp_extinction;
+    double* partial;               // 4 per task
+    double* group_sums;            // 4 per group
+    int* arrived;                  // per instance, then per group: rows written so far; 0 between launches
+    double* obs_row;
+};
+
 template <typename T>
 struct DetTileArgs {               // noise-off DP step over 64 x 32 tiles of every instance (a = it.R[k])
     const T* in;
@@ -126,16 +156,12 @@ cudaError_t launch_rk4<float>(const RK4Args<float>& a, bool det, int grid, cudaS
 template <>
 cudaError_t launch_rk4<double>(const RK4Args<double>& a, bool det, int grid, cudaStream_t s);
 template <typename T>
-cudaError_t launch_measure(const T* state, const InstTables& it, const int4* tasks, int n_tasks, int nf,
-                           double* partial, int grid, int block, cudaStream_t s, int spread = 0, int cx = -1,
-                           int cy = -1);
+cudaError_t launch_measure(const MeasureArgs<T>& a, int grid, int block, cudaStream_t s);
 template <typename T>
 cudaError_t launch_border_stop(const T* state, const InstTables& it, int n_inst, cudaStream_t s);
 template <typename T>
 cudaError_t launch_validate(const T* state, const InstTables& it, const int4* tasks, int n_tasks, int nf, int grid,
                             cudaStream_t s);
-cudaError_t launch_finalize(const double* partial, const int* task_begin, const InstTables& it, int n_inst, int nf,
-                            int dp_extinction, int spread, double* obs_row, cudaStream_t s);
 cudaError_t launch_consts(const double* a0, const double* astep, int n, int n_steps, double diff4, double sigma2, double dt,
                           const long long* step_base, long long step_off, Dc4* out, cudaStream_t s);
 cudaError_t launch_set_step(long long* d_step, long long v, cudaStream_t s);
