@@ -1,0 +1,35 @@
+"""FP32 draw: Poisson means through every length of the unrolled search and past its end,
+and boosted shapes down to where 1/k and U^(1/k) leave the normal range.  Bit for bit
+against the oracle."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("sampler", [0, 1])
+@pytest.mark.parametrize("dt,lo,hi", [(0.1, -3, 0.6), (0.06, -0.5, 0.2), (0.1, -30, -1)],
+                         ids=["m-to-60", "around-32", "tiny-shapes"])
+def test_fp32_draw_matches_oracle(oracle, dt, lo, hi, sampler):
+    import trophic_maelstorm_gb300 as tmg
+    rng = np.random.default_rng(17)
+    ctx = tmg.Context(0)
+    Ls = [33, 96, 257]
+    model = tmg.dp_model(dt=dt, sampler=sampler)
+    init = []
+    for L in Ls:
+        f = (10.0 ** rng.uniform(lo, hi, (L, L))).astype(np.float32)
+        f[rng.random((L, L)) < 0.3] = 0.0
+        init.append(f)
+    b = tmg.Batch(ctx, model, tmg.instances(Ls, [2 + k for k in range(len(Ls))], 0.53), tmg.TM_FP32)
+    b.upload(init)
+    _, st = b.advance(4, [])
+    fin = b.download()
+    b.close()
+    ctx.close()
+    for k, L in enumerate(Ls):
+        p = oracle.DPParams(0.53, 0.0, model.b, model.c, model.D, model.sigma, model.dt, model.dx, model.clamp_lo,
+                            model.clamp_eps, model.remainder, model.sampler)
+        _, _, want, ost = oracle.dp_run(p, init[k], 2 + k, 4, [4])
+        assert np.array_equal(fin[k], want), (k, L)
+        assert st[k] == ost
