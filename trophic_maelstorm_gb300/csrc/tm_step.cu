@@ -77,7 +77,8 @@ __device__ __forceinline__ float finish_site(const DornicArgs<float>& A, float r
     }
     if (REM != 2) {
         if (res < A.ceps && res >= A.clo) res = 0.0f;
-        st |= value_status(res);
+        // one test where nothing is to report: NaN, Inf and anything with a sign bit lie above
+        if (__float_as_uint(res) >= 0x7f800000u) st |= value_status(res);
     }
     return res;
 }
@@ -116,9 +117,11 @@ __global__ void __launch_bounds__(256, 4) dornic_step_kernel(const DornicArgs<fl
     const int cap = A.rows_cap * 32;
     unsigned char* wbase = smem_raw + (threadIdx.x >> 5) * warp_scratch_bytes(A.rows_cap);
     float* const Wres = reinterpret_cast<float*>(wbase);
-    float* const Wqm = Wres + cap;
-    float* const Wqmu = Wqm + cap;
-    unsigned short* const Wqi = reinterpret_cast<unsigned short*>(Wqmu + cap);
+    // Poisson mean and Gamma shape as one word pair, stores by the 32-bit site index and one
+    // test for the status bits: a dozen issue slots of the 400 a drawn chunk takes (fully
+    // active sweep, 40 steps: 57.96 -> 57.19 ms)
+    float2* const Wq = reinterpret_cast<float2*>(Wres + cap);
+    unsigned short* const Wqi = reinterpret_cast<unsigned short*>(Wq + cap);
     unsigned* const Wrows = defer_rows[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
@@ -197,8 +200,7 @@ __global__ void __launch_bounds__(256, 4) dornic_step_kernel(const DornicArgs<fl
                 if (live) {
                     const int pos = nq + __popc(bal & lt_mask);
                     Wqi[pos] = (unsigned short)(r * 32 + lane);
-                    Wqm[pos] = pm * cur;
-                    Wqmu[pos] = alpha * A.two_s2;
+                    Wq[pos] = make_float2(pm * cur, alpha * A.two_s2);
                 }
                 nq += __popc(bal);
                 north = cur;
@@ -216,15 +218,14 @@ __global__ void __launch_bounds__(256, 4) dornic_step_kernel(const DornicArgs<fl
                 if (has) {
                     const int li = Wqi[j];
                     const uint32_t site = site_index(y0 + (li >> 5), L, x0 + (li & 31));
-                    const float v = dornic_draw_fast(seed, site, step, Wqm[j], Wqmu[j], inv_lambda, SAMP, tab,
-                                                     deferred);
+                    const float2 q = Wq[j];
+                    const float v = dornic_draw_fast(seed, site, step, q.x, q.y, inv_lambda, SAMP, tab, deferred);
                     if constexpr (kStoreEarly) {
                         if (!deferred) {
-                            const long long o = (long long)(y0 + (li >> 5)) * L + x0 + (li & 31);
                             float res = v;
                             if (!(A.zero_fixed && is_pos_zero(v)))
-                                res = finish_site<REM>(A, v, sb ? sb[o] : A.b, st);
-                            dst[o] = res;
+                                res = finish_site<REM>(A, v, sb ? sb[site] : A.b, st);
+                            dst[site] = res;
                         }
                     } else {
                         if (deferred) atomicOr(Wrows + (li & 31), 1u << (li >> 5));
@@ -237,7 +238,7 @@ __global__ void __launch_bounds__(256, 4) dornic_step_kernel(const DornicArgs<fl
                     const int li = Wqi[j];
                     A.dlist[(long long)gw * A.seg_cap + nseg + __popc(bal & lt_mask)] =
                         make_uint4((unsigned)k, site_index(y0 + (li >> 5), L, x0 + (li & 31)),
-                                   __float_as_uint(Wqm[j]), __float_as_uint(Wqmu[j]));
+                                   __float_as_uint(Wq[j].x), __float_as_uint(Wq[j].y));
                 }
                 nseg += __popc(bal);
             }
