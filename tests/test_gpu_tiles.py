@@ -72,3 +72,30 @@ def test_reciprocal_range_matches_oracle(oracle, precision, planted):
     with np.errstate(all="ignore"):
         want = _off_step(oracle, m, 0.9, f0)
     assert np.array_equal(fin, want, equal_nan=True)
+
+
+@pytest.mark.parametrize("precision", [0, 1], ids=["fp64", "fp32"])
+@pytest.mark.parametrize("L", [31, 64, 129])
+def test_tile_status_bits(L, precision):
+    """A step size far above the stability bound: O goes negative, then overflows; the
+    status bits are those of the fields that the tiles stored, each step."""
+    import trophic_maelstorm_gb300 as tmg
+    dtype = np.float64 if precision == 0 else np.float32
+    ctx = tmg.Context(0)
+    rng = np.random.default_rng(3)
+    b = tmg.Batch(ctx, tmg.rietkerk_model(dt=0.05, deterministic=1), tmg.instances([L, L], [4, 5], 0.9), precision)
+    calm = np.stack([np.zeros((L, L)), np.ones((L, L)), np.ones((L, L))]).astype(dtype)
+    wild = np.stack([rng.uniform(0, 1, (L, L)), np.full((L, L), 0.5), 1.0 + rng.uniform(-0.1, 0.1, (L, L))]).astype(dtype)
+    b.upload([calm, wild])
+    want = [0, 0]
+    seen = 0
+    with np.errstate(all="ignore"):
+        for _ in range(100):
+            _, st = b.advance(1, [])
+            for k, f in enumerate(b.download()):
+                want[k] |= (0 if np.all(np.isfinite(f)) else 0x1) | (0x2 if np.any(f < 0) else 0)
+                assert int(st[k]) == want[k]
+            seen |= want[1]
+    b.close()
+    ctx.close()
+    assert seen == 0x3
