@@ -1,13 +1,12 @@
-// tm_rk4.cu -- RK4 of the Rietkerk three-field right-hand side, fused in one
-// pass over a shared-memory tile, and the noise-off DP stage kernels.
+// tm_rk4.cu -- RK4 of the Rietkerk three-field right-hand side in FP64, fused in one
+// pass over a shared-memory tile (tm_rk4_f32.cu: FP32), and the noise-off DP step's tiles.
 //
 // Rietkerk (rietkerk_bjork_FKE.cpp:2363-2444 stochastic remainder f_2Dor,
 // :1760-1856 noise-off f_2D): the W and O tendencies carry 5-point
 // Laplacians, so stage s needs stage s-1 values one site further out.  A CTA
-// loads a (64+8) x (32+8) region of [P*, W, O] (halo 4, periodic wrap) into
-// shared memory and runs all four stages there, stage s only on the region
-// inset by s+1 cells, so the 64 x 32 interior comes out exact after stage 4
-// with 1.15 stage evaluations per cell and stage.
+// loads a region of [P*, W, O] with a halo of 4 (periodic wrap) into shared memory
+// and runs all four stages there, stage s only on the region inset by s+1 cells, so
+// the interior (64 columns by 24 or 12 rows) comes out exact after stage 4.
 // The state is read and written once per step (plus the halo re-read, which
 // hits L2); the K1..K4 temporaries the reference keeps as full lattices
 // never leave the SM.
@@ -27,8 +26,7 @@ __device__ __forceinline__ T add_pow2_times(T c, T s, T x)
 // One CTA per tile (persistent over tiles).  Stage s (0..3) is evaluated on
 // the region inset by s+1 cells -- exactly the cells whose stage-s value an
 // interior cell depends on -- so the interior is exact after stage 3.  Stage
-// inputs ping-pong between two shared buffers, so each stage needs one barrier
-// and no value is held in registers across it.
+// inputs ping-pong between two shared buffers, so each stage needs one barrier.
 // Tile rows by bulk copy: for a tile that does not wrap in x on a lattice whose rows
 // are multiples of 16 bytes, each of the halo rows is a contiguous segment of RK_RX
 // values starting on a 16-byte boundary (instance offsets and field strides are

@@ -15,7 +15,7 @@
 // The whole warp runs the straight-line draw together (lanes without a site repeat
 // one): lanes that left the search one by one made the rest of the draw run twice.
 // Measured, 16 lattices of 256^2, 32 steps of a decaying run: RK4 remainder 20.2 ->
-// 4.4 ms; general sampler for every site 319 FP64 instructions per 32 sites, now about 30
+// 3.9 ms; general sampler for every site 319 FP64 instructions per 32 sites, now about 30
 // (Euler-exact remainder).  Bound by the FP64 pipe (60-65 % busy) and the integer
 // pipe together.  Two CTAs of 8 warps per SM: three (80 registers, small spills) took
 // the same time, four 13 % more.
