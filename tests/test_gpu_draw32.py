@@ -33,3 +33,27 @@ def test_fp32_draw_matches_oracle(oracle, dt, lo, hi, sampler):
         _, _, want, ost = oracle.dp_run(p, init[k], 2 + k, 4, [4])
         assert np.array_equal(fin[k], want), (k, L)
         assert st[k] == ost
+
+
+@pytest.mark.parametrize("n", [1, 30])
+def test_fp32_default_rows_do_not_change_the_fields(n):
+    """A batch large enough for 16-row tasks, and one below: the same bits as 8-row and 5-row tasks."""
+    import trophic_maelstorm_gb300 as tmg
+    rng = np.random.default_rng(23)
+    ctx = tmg.Context(0)
+    Ls = [513] * n + [40]
+    init = [(rng.uniform(0.0, 2.0, (L, L)) * (rng.random((L, L)) < 0.5)).astype(np.float32) for L in Ls]
+    got = []
+    for rows in (0, 8, 5):
+        b = tmg.Batch(ctx, tmg.dp_model(dt=0.1), tmg.instances(Ls, list(range(len(Ls))), 0.53), tmg.TM_FP32)
+        if rows:
+            b.set_launch(rows, 0)
+        elif n == 30:
+            assert b.get_launch()[0] == 16
+        b.upload(init)
+        b.advance(3, [])
+        got.append(b.download())
+        b.close()
+    ctx.close()
+    for k in range(len(Ls)):
+        assert np.array_equal(got[0][k], got[1][k]) and np.array_equal(got[0][k], got[2][k])

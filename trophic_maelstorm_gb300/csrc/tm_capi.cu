@@ -130,18 +130,26 @@ void free_graphs(tm_batch* b)
 // FP64 sites take tens of times longer to draw, so its tasks are cut finer: four for
 // each of the 16 warps that an SM holds (16 lattices of 256^2: 4.4 ms for 32 steps
 // against 4.6 with two per warp and 5.6 with 8-row tasks).
+// FP32 DP batches take 16 rows where that still leaves three tasks for each of the 32
+// warps that an SM holds: fewer rows read twice and fewer task starts (40 steps of an 89
+// M-site sweep 57.2 against 55.6 ms; 32 lattices of 512^2 168 against 161 us a step), but
+// 1.7 tasks per warp leave warps idle (4 lattices of 1024^2: 84 against 95 us).  The
+// Rietkerk draw's queue is larger and 16 rows of it fit an SM three times only: 8 rows.
 int default_rows(const tm_batch* b)
 {
-    const long long want = (b->precision == TM_FP64 ? 4LL * 16 : 2LL * 4) * std::max(1, b->ctx->num_sms);
-    int R = 8;
-    for (; R > 1; R >>= 1) {
+    const long long sms = std::max(1, b->ctx->num_sms);
+    const long long want = (b->precision == TM_FP64 ? 4LL * 16 : 2LL * 4) * sms;
+    const auto tasks = [b](int R) {
         long long n = 0;
         for (int k = 0; k < b->n_inst; ++k) {
             const long long L = b->inst[k].L;
             n += ((L + R - 1) / R) * ((L + 31) / 32);
         }
-        if (n >= want) break;
-    }
+        return n;
+    };
+    if (b->precision == TM_FP32 && b->model == 0 && tasks(16) >= 3 * 32 * sms) return 16;
+    int R = 8;
+    while (R > 1 && tasks(R) < want) R >>= 1;
     return R;
 }
 

@@ -43,9 +43,9 @@ __device__ __forceinline__ float rem_f(float x, float b, float c, int cubic)
 // of every site (res), and the queue of live sites (Poisson mean, shape, index).
 constexpr int kWarps = 8;
 
-__host__ __device__ __forceinline__ size_t warp_scratch_bytes(int rows_cap)
+__host__ __device__ __forceinline__ size_t warp_scratch_bytes(int rows_cap, bool keep_res)
 {
-    return (size_t)rows_cap * 32 * (3 * sizeof(float) + sizeof(unsigned short));
+    return (size_t)rows_cap * 32 * ((keep_res ? 3 : 2) * sizeof(float) + sizeof(unsigned short));
 }
 
 __device__ __forceinline__ bool is_pos_zero(float x) { return __float_as_uint(x) == 0u; }
@@ -115,12 +115,12 @@ __global__ void __launch_bounds__(256, 4) dornic_step_kernel(const DornicArgs<fl
     pdl_wait();
     __syncthreads();
     const int cap = A.rows_cap * 32;
-    unsigned char* wbase = smem_raw + (threadIdx.x >> 5) * warp_scratch_bytes(A.rows_cap);
-    float* const Wres = reinterpret_cast<float*>(wbase);
+    unsigned char* wbase = smem_raw + (threadIdx.x >> 5) * warp_scratch_bytes(A.rows_cap, REM == 2);
+    float* const Wres = reinterpret_cast<float*>(wbase);                       // REM = 2 only
     // Poisson mean and Gamma shape as one word pair, stores by the 32-bit site index and one
     // test for the status bits: a dozen issue slots of the 400 a drawn chunk takes (fully
     // active sweep, 40 steps: 57.96 -> 57.19 ms)
-    float2* const Wq = reinterpret_cast<float2*>(Wres + cap);
+    float2* const Wq = reinterpret_cast<float2*>(Wres + (REM == 2 ? cap : 0));
     unsigned short* const Wqi = reinterpret_cast<unsigned short*>(Wq + cap);
     unsigned* const Wrows = defer_rows[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
@@ -298,7 +298,7 @@ cudaError_t launch_dornic_t(const DornicArgs<float>& a, int grid, int block, siz
 {
     static bool attr_set = false;
     if (!attr_set) {
-        const int full = (int)(warp_scratch_bytes(kMaxRowsPerTask) * kWarps);
+        const int full = (int)(warp_scratch_bytes(kMaxRowsPerTask, REM == 2) * kWarps);
         const cudaError_t e = cudaFuncSetAttribute(dornic_step_kernel<REM, SAMP, CAP>,
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, full);
         if (e != cudaSuccess) return e;
@@ -333,7 +333,7 @@ cudaError_t launch_dornic<float>(const DornicArgs<float>& a, int rem, int grid, 
 {
     if (a.n_tasks <= 0) return cudaSuccess;
     if (block != 32 * kWarps || a.rows_cap < 1 || a.rows_cap > kMaxRowsPerTask) return cudaErrorInvalidValue;
-    const size_t smem = warp_scratch_bytes(a.rows_cap) * kWarps;
+    const size_t smem = warp_scratch_bytes(a.rows_cap, rem == 2) * kWarps;
     if (rem == 0) return launch_dornic_r<0>(a, grid, block, smem, s);
     if (rem == 1) return launch_dornic_r<1>(a, grid, block, smem, s);
     if (rem == 2) return launch_dornic_r<2>(a, grid, block, smem, s);
