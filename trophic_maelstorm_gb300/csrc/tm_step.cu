@@ -11,11 +11,9 @@
 // a straight-line path first; the few sites it defers (a few % of live sites)
 // go to the warp's own segment of a batch-wide list (no atomics: the warp keeps
 // the count) that a second kernel draws with the general sampler, so the step
-// kernel's loop body holds no general-sampler code.  The FP32 DP step stores
-// each site as soon as its value is known: absorbing sites while the rows
-// stream in (pass 1), drawn sites right after their draw (pass 2).  The
-// Rietkerk draw keeps a third pass that stores from shared memory.  Per site it
-// fuses:
+// kernel's loop body holds no general-sampler code.  Each site is stored as soon
+// as its value is known: absorbing sites while the rows stream in (pass 1), drawn
+// sites right after their draw (pass 2).  Per site it fuses:
 //   alpha_i  = (D/dx^2) * sum of the 4 neighbours       stochasticSPDP.cpp:1037-1038
 //   skip     if alpha_i == 0 and rho_i == 0             :1049-1052
 //   rho*     = Gamma(2 alpha_i/sigma^2 + Poisson(lambda e^{beta dt} rho_i)) / lambda   :1053-1059
@@ -39,13 +37,13 @@ __device__ __forceinline__ float rem_f(float x, float b, float c, int cubic)
     return f;
 }
 
-// Per-warp shared scratch for one task of up to rows_cap rows: the Dornic draw
-// of every site (res), and the queue of live sites (Poisson mean, shape, index).
+// Per-warp shared scratch for one task of up to rows_cap rows: the queue of live sites
+// (Poisson mean, shape, index).
 constexpr int kWarps = 8;
 
-__host__ __device__ __forceinline__ size_t warp_scratch_bytes(int rows_cap, bool keep_res)
+__host__ __device__ __forceinline__ size_t warp_scratch_bytes(int rows_cap)
 {
-    return (size_t)rows_cap * 32 * ((keep_res ? 3 : 2) * sizeof(float) + sizeof(unsigned short));
+    return (size_t)rows_cap * 32 * (2 * sizeof(float) + sizeof(unsigned short));
 }
 
 __device__ __forceinline__ bool is_pos_zero(float x) { return __float_as_uint(x) == 0u; }
@@ -110,19 +108,16 @@ __global__ void __launch_bounds__(256, 4) dornic_step_kernel(const DornicArgs<fl
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ SmemTab<float> tab;
-    __shared__ unsigned defer_rows[kWarps][32];
     tab.fill();
     pdl_wait();
     __syncthreads();
     const int cap = A.rows_cap * 32;
-    unsigned char* wbase = smem_raw + (threadIdx.x >> 5) * warp_scratch_bytes(A.rows_cap, REM == 2);
-    float* const Wres = reinterpret_cast<float*>(wbase);                       // REM = 2 only
+    unsigned char* wbase = smem_raw + (threadIdx.x >> 5) * warp_scratch_bytes(A.rows_cap);
     // Poisson mean and Gamma shape as one word pair, stores by the 32-bit site index and one
     // test for the status bits: a dozen issue slots of the 400 a drawn chunk takes (fully
     // active sweep, 40 steps: 57.96 -> 57.19 ms)
-    float2* const Wq = reinterpret_cast<float2*>(Wres + (REM == 2 ? cap : 0));
+    float2* const Wq = reinterpret_cast<float2*>(wbase);
     unsigned short* const Wqi = reinterpret_cast<unsigned short*>(Wq + cap);
-    unsigned* const Wrows = defer_rows[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
     const int gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
@@ -157,13 +152,7 @@ __global__ void __launch_bounds__(256, 4) dornic_step_kernel(const DornicArgs<fl
             float south = act ? src[(long long)((y0 == L - 1) ? 0 : y0 + 1) * L + x] : 0.0f;
             int nq = 0;
             unsigned st = 0;
-            // The DP step finishes and stores every site where its value is known:
-            // absorbing and noise-off sites in pass 1, drawn sites in pass 2, so it has no
-            // pass 3 and no round trip of the draws through shared memory.  (For P* of the
-            // Rietkerk step the compiler then spills; it keeps the three passes.)
-            constexpr bool kStoreEarly = REM != 2;
-            const float* __restrict__ sb = (kStoreEarly && A.site_b) ? A.site_b + A.it.off[k] : nullptr;
-            if (!kStoreEarly) Wrows[lane] = 0u;
+            const float* __restrict__ sb = A.site_b ? A.site_b + A.it.off[k] : nullptr;
             for (int r = 0; r < rows; ++r) {
                 const int y = y0 + r;
                 float next = 0.0f;
@@ -183,19 +172,12 @@ __global__ void __launch_bounds__(256, 4) dornic_step_kernel(const DornicArgs<fl
                 const float alpha = A.dcoef * nsum;
                 const bool live = act && !(alpha == 0.0f && cur == 0.0f) && SAMP != 2;
                 const unsigned bal = __ballot_sync(0xffffffffu, live);
-                if (!live) {
-                    if constexpr (kStoreEarly) {
-                        if (act) {
-                            const float rs = (SAMP == 2) ? a1 * cur + a2 * alpha : 0.0f;
-                            const long long o = (long long)y * L + x;
-                            float res = rs;
-                            if (!(A.zero_fixed && is_pos_zero(rs)))
-                                res = finish_site<REM>(A, rs, sb ? sb[o] : A.b, st);
-                            dst[o] = res;
-                        }
-                    } else {
-                        Wres[r * 32 + lane] = (SAMP == 2 && act) ? a1 * cur + a2 * alpha : 0.0f;
-                    }
+                if (!live && act) {
+                    const float rs = (SAMP == 2) ? a1 * cur + a2 * alpha : 0.0f;
+                    const long long o = (long long)y * L + x;
+                    float res = rs;
+                    if (!(A.zero_fixed && is_pos_zero(rs))) res = finish_site<REM>(A, rs, sb ? sb[o] : A.b, st);
+                    dst[o] = res;
                 }
                 if (live) {
                     const int pos = nq + __popc(bal & lt_mask);
@@ -220,16 +202,10 @@ __global__ void __launch_bounds__(256, 4) dornic_step_kernel(const DornicArgs<fl
                     const uint32_t site = site_index(y0 + (li >> 5), L, x0 + (li & 31));
                     const float2 q = Wq[j];
                     const float v = dornic_draw_fast(seed, site, step, q.x, q.y, inv_lambda, SAMP, tab, deferred);
-                    if constexpr (kStoreEarly) {
-                        if (!deferred) {
-                            float res = v;
-                            if (!(A.zero_fixed && is_pos_zero(v)))
-                                res = finish_site<REM>(A, v, sb ? sb[site] : A.b, st);
-                            dst[site] = res;
-                        }
-                    } else {
-                        if (deferred) atomicOr(Wrows + (li & 31), 1u << (li >> 5));
-                        else Wres[li] = v;
+                    if (!deferred) {
+                        float res = v;
+                        if (!(A.zero_fixed && is_pos_zero(v))) res = finish_site<REM>(A, v, sb ? sb[site] : A.b, st);
+                        dst[site] = res;
                     }
                 }
                 // deferred sites: appended to this warp's segment of the list
@@ -243,24 +219,6 @@ __global__ void __launch_bounds__(256, 4) dornic_step_kernel(const DornicArgs<fl
                 nseg += __popc(bal);
             }
             __syncwarp();
-            [[maybe_unused]] unsigned drows = 0;   // rows of this lane's column left to the general sampler
-            if constexpr (!kStoreEarly) drows = Wrows[lane];
-            // pass 3: remainder, clamp, store (sites left to the general sampler
-            // are finished and stored by it).  When zero_fixed holds a +0 draw --
-            // every absorbing site -- finishes as +0 and skips the arithmetic.
-            if (!kStoreEarly && act) {
-                const float* __restrict__ sb3 = A.site_b ? A.site_b + A.it.off[k] : nullptr;
-                for (int r = 0; r < rows; ++r) {
-                    if ((drows >> r) & 1u) continue;
-                    const float rs = Wres[r * 32 + lane];
-                    float res = rs;
-                    if (!(A.zero_fixed && is_pos_zero(rs))) {
-                        const float bi = sb3 ? sb3[(long long)(y0 + r) * L + x] : A.b;
-                        res = finish_site<REM>(A, rs, bi, st);
-                    }
-                    dst[(long long)(y0 + r) * L + x] = res;
-                }
-            }
             if (st) atomicOr(A.it.status + k, st);
         }
         __syncwarp();
@@ -298,7 +256,7 @@ cudaError_t launch_dornic_t(const DornicArgs<float>& a, int grid, int block, siz
 {
     static bool attr_set = false;
     if (!attr_set) {
-        const int full = (int)(warp_scratch_bytes(kMaxRowsPerTask, REM == 2) * kWarps);
+        const int full = (int)(warp_scratch_bytes(kMaxRowsPerTask) * kWarps);
         const cudaError_t e = cudaFuncSetAttribute(dornic_step_kernel<REM, SAMP, CAP>,
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, full);
         if (e != cudaSuccess) return e;
@@ -333,7 +291,7 @@ cudaError_t launch_dornic<float>(const DornicArgs<float>& a, int rem, int grid, 
 {
     if (a.n_tasks <= 0) return cudaSuccess;
     if (block != 32 * kWarps || a.rows_cap < 1 || a.rows_cap > kMaxRowsPerTask) return cudaErrorInvalidValue;
-    const size_t smem = warp_scratch_bytes(a.rows_cap, rem == 2) * kWarps;
+    const size_t smem = warp_scratch_bytes(a.rows_cap) * kWarps;
     if (rem == 0) return launch_dornic_r<0>(a, grid, block, smem, s);
     if (rem == 1) return launch_dornic_r<1>(a, grid, block, smem, s);
     if (rem == 2) return launch_dornic_r<2>(a, grid, block, smem, s);
