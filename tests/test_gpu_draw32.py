@@ -57,3 +57,24 @@ def test_fp32_default_rows_do_not_change_the_fields(n):
     ctx.close()
     for k in range(len(Ls)):
         assert np.array_equal(got[0][k], got[1][k]) and np.array_equal(got[0][k], got[2][k])
+
+
+def test_fp32_list_grows_with_the_grid():
+    """More blocks per SM than a batch was created for: its list of deferred sites is laid out again."""
+    import trophic_maelstorm_gb300 as tmg
+    rng = np.random.default_rng(29)
+    ctx = tmg.Context(0)
+    f = rng.uniform(0.0, 2.0, (700, 700)).astype(np.float32)
+    got = []
+    for launches in ([], [(1, 0), (0, 64), (0, 2)], [(1, 64)]):
+        b = tmg.Batch(ctx, tmg.dp_model(dt=0.1), tmg.instances([700], [3], 0.53), tmg.TM_FP32)
+        b.upload([f])
+        b.advance(1, [])
+        for rows, ctas in launches:
+            b.set_launch(rows, ctas)
+            b.advance(1, [])
+        b.advance(4 - 1 - len(launches), [])
+        got.append(b.download()[0])
+        b.close()
+    ctx.close()
+    assert np.array_equal(got[0], got[2]) and np.array_equal(got[0], got[1])

@@ -124,6 +124,16 @@ void free_graphs(tm_batch* b)
     }
 }
 
+long long count_tasks(const tm_batch* b, int rows)
+{
+    long long n = 0;
+    for (int k = 0; k < b->n_inst; ++k) {
+        const long long L = b->inst[k].L;
+        n += ((L + rows - 1) / rows) * ((L + 31) / 32);
+    }
+    return n;
+}
+
 // Rows per warp task for a new batch: 8, or fewer when the batch is too small
 // to give every scheduler of the GPU two tasks (one 128^2 lattice is 64 tasks of
 // 8 rows).  The results do not depend on the task shape.
@@ -139,17 +149,9 @@ int default_rows(const tm_batch* b)
 {
     const long long sms = std::max(1, b->ctx->num_sms);
     const long long want = (b->precision == TM_FP64 ? 4LL * 16 : 2LL * 4) * sms;
-    const auto tasks = [b](int R) {
-        long long n = 0;
-        for (int k = 0; k < b->n_inst; ++k) {
-            const long long L = b->inst[k].L;
-            n += ((L + R - 1) / R) * ((L + 31) / 32);
-        }
-        return n;
-    };
-    if (b->precision == TM_FP32 && b->model == 0 && tasks(16) >= 3 * 32 * sms) return 16;
+    if (b->precision == TM_FP32 && b->model == 0 && count_tasks(b, 16) >= 3 * 32 * sms) return 16;
     int R = 8;
-    while (R > 1 && tasks(R) < want) R >>= 1;
+    while (R > 1 && count_tasks(b, R) < want) R >>= 1;
     return R;
 }
 
@@ -178,12 +180,19 @@ int rk64_tile_rows(const tm_batch* b)
     return best;
 }
 
+// Warps of the FP32 step's grid at most, each with a segment of the deferred-site list.
+long long list_segments(const tm_batch* b)
+{
+    return std::min<long long>((long long)b->n_tasks + 8, (long long)std::max(1, b->ctx->num_sms) * std::max(b->ctas_per_sm, 4) * 8);
+}
+
 int build_tasks(tm_batch* b)
 {
     // warp tasks
     std::vector<int4> tasks;
     std::vector<int> begin(b->n_inst + 1, 0);
     const int R = b->rows_per_task;
+    tasks.reserve((size_t)count_tasks(b, R));
     for (int k = 0; k < b->n_inst; ++k) {
         begin[k] = (int)tasks.size();
         const int L = b->inst[k].L;
@@ -196,13 +205,14 @@ int build_tasks(tm_batch* b)
     cudaFree(b->d_partial); b->d_partial = nullptr;
     b->n_tasks = (int)tasks.size();
     TM_CUDA(dalloc(&b->d_tasks, tasks.size()));
-    // partials and group sums (four numbers each), then the arrival counters
+    // partials and group sums, four numbers each; the arrival counters follow the table of
+    // first tasks, whose upload sets them to 0
     b->n_groups = measure_group_base(b->n_tasks, b->n_inst) + 1;
-    const size_t rows = 4 * (tasks.size() + b->n_groups), counters = (size_t)b->n_inst + b->n_groups;
-    TM_CUDA(dalloc(&b->d_partial, rows + (counters + 1) / 2));
-    TM_CUDA(cudaMemset(b->d_partial + rows, 0, counters * sizeof(int)));
+    TM_CUDA(dalloc(&b->d_partial, 4 * (tasks.size() + b->n_groups)));
+    begin.resize((size_t)b->n_inst + 1 + b->n_inst + b->n_groups, 0);
     TM_CUDA(cudaMemcpy(b->d_tasks, tasks.data(), tasks.size() * sizeof(int4), cudaMemcpyHostToDevice));
-    if (!b->d_task_begin) TM_CUDA(dalloc(&b->d_task_begin, begin.size()));
+    cudaFree(b->d_task_begin); b->d_task_begin = nullptr;
+    TM_CUDA(dalloc(&b->d_task_begin, begin.size()));
     TM_CUDA(cudaMemcpy(b->d_task_begin, begin.data(), begin.size() * sizeof(int), cudaMemcpyHostToDevice));
     // 64 x 32 tiles (Rietkerk RK4, noise-off DP; FP64 Rietkerk: rk64_tile_rows)
     if ((b->model == 1 || b->dpm.deterministic) && !b->d_btasks) {
@@ -219,11 +229,11 @@ int build_tasks(tm_batch* b)
     }
     if (b->precision == TM_FP32) {
         // the deferred-site list: a step grid of nw warps gives every warp a segment of
-        // ceil(n_tasks / nw) tasks' sites, nw * that <= (n_tasks + nw) * R * 32 entries;
-        // sized for the largest grid (64 CTAs of 8 warps per SM, at most one warp per task)
+        // ceil(n_tasks / nw) tasks' sites, nw * that <= (n_tasks + nw) * R * 32 entries; sized
+        // for the grid of ctas_per_sm (the default's at least), at most one warp per task
         cudaFree(b->d_dlist); b->d_dlist = nullptr;
         cudaFree(b->d_dcnt); b->d_dcnt = nullptr;
-        b->max_seg = std::min<long long>((long long)b->n_tasks + 8, (long long)std::max(1, b->ctx->num_sms) * 64 * 8);
+        b->max_seg = list_segments(b);
         b->dlist_cap = ((long long)b->n_tasks + b->max_seg) * R * 32;
         TM_CUDA(dalloc(&b->d_dlist, (size_t)b->dlist_cap));
         TM_CUDA(dalloc(&b->d_dcnt, (size_t)b->max_seg));
@@ -419,7 +429,7 @@ int measure_as(tm_batch* b, int j)
     a.dp_extinction = b->model == 0;
     a.partial = b->d_partial;
     a.group_sums = b->d_partial + 4LL * b->n_tasks;
-    a.arrived = (int*)(a.group_sums + 4LL * b->n_groups);
+    a.arrived = b->d_task_begin + b->n_inst + 1;
     a.obs_row = b->d_obs + (size_t)j * b->n_inst * obs_w(b);
     TM_CUDA(launch_measure<T>(a, warp_grid(b, b->n_tasks), 256, b->ctx->stream));
     return TM_OK;
@@ -840,7 +850,11 @@ int tm_batch_set_launch(tm_batch* b, int rows, int ctas)
     TM_CUDA(cudaStreamSynchronize(b->ctx->stream));
     bool rebuild = false;
     if (rows > 0 && rows != b->rows_per_task) { b->rows_per_task = rows; rebuild = true; }
-    if (ctas > 0 && ctas != b->ctas_per_sm) { b->ctas_per_sm = ctas; free_graphs(b); }
+    if (ctas > 0 && ctas != b->ctas_per_sm) {
+        b->ctas_per_sm = ctas;
+        free_graphs(b);
+        if (b->precision == TM_FP32 && list_segments(b) > b->max_seg) rebuild = true;
+    }
     return rebuild ? build_tasks(b) : TM_OK;
 }
 
