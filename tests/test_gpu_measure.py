@@ -89,3 +89,33 @@ def test_spreading_sums(precision, rows):
             assert obs[0, k, 2] == int(((y - 7) ** 2 + (x - 5) ** 2).sum())
     b.close()
     ctx.close()
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_ramp_across_measurements_matches_oracle(oracle, precision):
+    """A ramp's constants are queued for runs of steps that measurements, graphs and calls cut differently."""
+    import trophic_maelstorm_gb300 as tmg
+    rng = np.random.default_rng(9)
+    ctx = tmg.Context(0)
+    prec, dtype = (tmg.TM_FP32, np.float32) if precision == "fp32" else (tmg.TM_FP64, np.float64)
+    L, a, a_step, n = 33, 0.72, -3e-4, 150
+    model = tmg.dp_model(dt=0.1)
+    init = rng.uniform(0.5, 1.5, (L, L)).astype(dtype)
+    p = oracle.DPParams(a, a_step, model.b, model.c, model.D, model.sigma, model.dt, model.dx, model.clamp_lo, model.clamp_eps,
+                        model.remainder, model.sampler)
+    meas = [1, 2, 3, 20, 31, 32, 33, 66, 100, 101, 140, 150]
+    mean, active, want, _ = oracle.dp_run(p, init, 5, n, meas)
+    for calls in ([n], [1, 40, 5, 104]):
+        b = tmg.Batch(ctx, model, tmg.instances([L, L], [4, 5], a, a_step), prec)
+        b.upload([init, init])
+        got, at = [], 0
+        for steps in calls:
+            now = [m for m in meas if at < m <= at + steps]
+            obs, _ = b.advance(steps, now)
+            got += [obs[j, 1] for j in range(len(now))]
+            at += steps
+        assert np.array_equal(b.download()[1], want)
+        b.close()
+        for j in range(len(meas)):
+            assert abs(got[j][0] - mean[j]) <= 1e-12 * mean[j] and got[j][1] == active[j]
+    ctx.close()
