@@ -11,8 +11,8 @@
 //
 // A measurement is short beside its launches and round trips.  With a second kernel of
 // one warp per instance for the sums, 64 spreading FP64 lattices of 101 x 101 took 18.7 us
-// to measure, and 12.8 us with the sums in the same launch (and no additions for rows of
-// zeros); on a 4096 x 4096 FP32 Rietkerk lattice that one warp walked 65,536 partials, 613
+// to measure, 12.8 us with the sums in the same launch (and no additions for rows of
+// zeros), 8.6 us with one-field code of its own (64 registers instead of 102); on a 4096 x 4096 FP32 Rietkerk lattice that one warp walked 65,536 partials, 613
 // us of a run of 24 steps and one measurement that went from 12.31 to 11.75 ms.
 //
 // GB300's FP64 rate is a small fraction of its FP32 rate, so the per-site work
@@ -155,15 +155,16 @@ __device__ __forceinline__ void observe(const MeasureArgs<T>& A, int k, const Su
 }
 
 // A warp takes a run of consecutive tasks, so that it reports a stretch of rows at a time.
-template <typename T>
+// NF fields: one field's code needs half the registers of three.
+template <typename T, int NF>
 __global__ void __launch_bounds__(256) measure_kernel(const MeasureArgs<T> A)
 {
     const int lane = threadIdx.x & 31;
     const long long gw = (long long)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int nw = (int)((gridDim.x * blockDim.x) >> 5);
     pdl_wait();
-    const int nf = A.nf, spread = A.spread;
-    const bool has1 = nf == 3 || spread, has2 = nf == 3;
+    const int spread = A.spread;
+    const bool has1 = NF == 3 || spread, has2 = NF == 3;
     const long long run = ((long long)A.n_tasks + nw - 1) / nw;
     const int end = (int)min((long long)A.n_tasks, (gw + 1) * run);
     int written = 0;                       // rows not reported yet
@@ -192,13 +193,13 @@ __global__ void __launch_bounds__(256) measure_kernel(const MeasureArgs<T> A)
                     const bool ok = in && r0 + j < tk.w;
                     const long long i = (long long)(tk.z + r0 + j) * L + x;
                     v0[j] = ok ? base[i] : T(0);
-                    v1[j] = (nf == 3 && ok) ? base[i + fs] : T(0);
-                    v2[j] = (nf == 3 && ok) ? base[i + 2 * fs] : T(0);
+                    v1[j] = (NF == 3 && ok) ? base[i + fs] : T(0);
+                    v2[j] = (NF == 3 && ok) ? base[i + 2 * fs] : T(0);
                 }
 #pragma unroll
                 for (int j = 0; j < kChunk; ++j) {
                     if (r0 + j >= tk.w) break;
-                    if (nf == 3) {
+                    if (NF == 3) {
                         c0.add(v0[j]);
                         any = true;
                         if (in) {
@@ -219,7 +220,7 @@ __global__ void __launch_bounds__(256) measure_kernel(const MeasureArgs<T> A)
         }
         const double s0 = any ? c0.warp_total() : 0.0;
         double s1 = 0.0, s2 = 0.0;
-        if (nf == 3) { s1 = c1.warp_total(); s2 = c2.warp_total(); }
+        if (NF == 3) { s1 = c1.warp_total(); s2 = c2.warp_total(); }
         if (spread && ac) {
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
@@ -265,7 +266,8 @@ template <typename T>
 cudaError_t launch_measure(const MeasureArgs<T>& a, int grid, int block, cudaStream_t s)
 {
     if (a.n_tasks <= 0) return cudaSuccess;
-    return launch_pdl(measure_kernel<T>, dim3(grid), dim3(block), 0, s, a);
+    if (a.nf == 3) return launch_pdl(measure_kernel<T, 3>, dim3(grid), dim3(block), 0, s, a);
+    return launch_pdl(measure_kernel<T, 1>, dim3(grid), dim3(block), 0, s, a);
 }
 template cudaError_t launch_measure<float>(const MeasureArgs<float>&, int, int, cudaStream_t);
 template cudaError_t launch_measure<double>(const MeasureArgs<double>&, int, int, cudaStream_t);
