@@ -70,6 +70,15 @@ __device__ __forceinline__ bool below(double a, double b)
 // 16 bits each (L <= 46340; kNowhere for a source without mass), and the largest shift.
 constexpr uint32_t kNowhere = 0xffffffffu;
 
+// How far t lies from c.  From L on the sources of a whole axis are looked at, so L stands
+// for more: an infinite velocity rounds to the largest int, and windows of that many
+// sites overflow.
+__device__ __forceinline__ int reach(int t, int c, int L)
+{
+    const long long d = (long long)t - c;
+    return (int)min(d < 0 ? -d : d, (long long)L);
+}
+
 template <typename T>
 __global__ void fke_prep_kernel(const T* rho, const T* vx, const T* vy, int L, T pref, T eps, T* w, uint32_t* to, int* smax)
 {
@@ -80,10 +89,10 @@ __global__ void fke_prep_kernel(const T* rho, const T* vx, const T* vy, int L, T
         const T rv = rho[i];
         const bool dead = below(rv, eps) || is_zero(rv);
         w[i] = dead ? T(0) : rv;
-        const int sx = round_int(to_float(ci, T(0)) + prod(vx[i], pref)) - ci;
-        const int sy = round_int(to_float(cj, T(0)) + prod(vy[i], pref)) - cj;
-        to[i] = dead ? kNowhere : ((uint32_t)pmod(ci + sx, L) << 16) | (uint32_t)pmod(cj + sy, L);
-        if (!dead) local = max(local, max(abs(sx), abs(sy)));
+        const int tx = round_int(to_float(ci, T(0)) + prod(vx[i], pref));
+        const int ty = round_int(to_float(cj, T(0)) + prod(vy[i], pref));
+        to[i] = dead ? kNowhere : ((uint32_t)pmod(tx, L) << 16) | (uint32_t)pmod(ty, L);
+        if (!dead) local = max(local, max(reach(tx, ci, L), reach(ty, cj, L)));
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) local = max(local, __shfl_xor_sync(0xffffffffu, local, o));
