@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "tm_per_device.h"
+
 // A context: one device and the stream every call on it launches on (tm_create).
 struct tm_ctx {
     int device = 0;
@@ -44,6 +46,17 @@ cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t 
     c.attrs = &a;
     c.numAttrs = 1;
     return cudaLaunchKernelEx(&c, kernel, static_cast<Params>(args)...);
+}
+
+// Lets `kernel` take `bytes` of dynamic shared memory on the current device; `done` is the
+// kernel's own.
+template <typename Kernel>
+cudaError_t allow_smem(PerDevice& done, Kernel kernel, size_t bytes)
+{
+    int device = 0;
+    const cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    return done.run(device, [&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); });
 }
 
 // Dornic constants of one instance: lambda e^{beta dt}, 1/lambda, e^{beta dt}, (e^{beta dt}-1)/beta

@@ -296,15 +296,11 @@ cudaError_t launch_rk4<double>(const RK4Args<double>& a, bool det, int grid, cud
 {
     if (a.n_tasks <= 0) return cudaSuccess;
     const size_t smem = 9 * (size_t)RK_RX * (RK64_TY + 2 * RK_H) * sizeof(double);   // of the tallest tile
-    static bool attr[2] = {false, false};
-    if (!attr[det ? 1 : 0]) {
-        const cudaError_t e =
-            det ? cudaFuncSetAttribute(rk4_tile64_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                : cudaFuncSetAttribute(rk4_tile64_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        attr[det ? 1 : 0] = true;
-    }
-    return launch_pdl(det ? rk4_tile64_kernel<true> : rk4_tile64_kernel<false>, dim3(grid), dim3(RK64_THREADS), smem, s, a);
+    static PerDevice allowed[2];
+    const auto kernel = det ? rk4_tile64_kernel<true> : rk4_tile64_kernel<false>;
+    const cudaError_t e = allow_smem(allowed[det ? 1 : 0], kernel, smem);
+    if (e != cudaSuccess) return e;
+    return launch_pdl(kernel, dim3(grid), dim3(RK64_THREADS), smem, s, a);
 }
 
 // ---- noise-off DP: drho/dt = a rho - b rho^2 - c rho^3 + D Lap(rho) ---------------
@@ -427,13 +423,9 @@ cudaError_t launch_det_t(const DetTileArgs<T>& a, int grid, cudaStream_t s)
 {
     constexpr int H = RAD * NST;
     const size_t smem = 3 * (size_t)(RK_TX + 2 * H) * (RK_TY + 2 * H) * sizeof(T);
-    static bool attr = false;
-    if (!attr) {
-        const cudaError_t e =
-            cudaFuncSetAttribute(dp_det_tile_kernel<T, RAD, NST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        attr = true;
-    }
+    static PerDevice allowed;
+    const cudaError_t e = allow_smem(allowed, dp_det_tile_kernel<T, RAD, NST>, smem);
+    if (e != cudaSuccess) return e;
     return launch_pdl(dp_det_tile_kernel<T, RAD, NST>, dim3(grid), dim3(RK_THREADS), smem, s, a);
 }
 

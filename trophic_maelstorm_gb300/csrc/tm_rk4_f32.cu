@@ -361,15 +361,11 @@ cudaError_t launch_rk4<float>(const RK4Args<float>& a, bool det, int grid, cudaS
 {
     if (a.n_tasks <= 0) return cudaSuccess;
     const size_t smem = 9 * (size_t)RK_RN * sizeof(float);
-    static bool attr[2] = {false, false};
-    if (!attr[det ? 1 : 0]) {
-        const cudaError_t e =
-            det ? cudaFuncSetAttribute(rk4_tile_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                : cudaFuncSetAttribute(rk4_tile_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        attr[det ? 1 : 0] = true;
-    }
-    return launch_pdl(det ? rk4_tile_kernel<true> : rk4_tile_kernel<false>, dim3(grid), dim3(RK_THREADS), smem, s, a);
+    static PerDevice allowed[2];
+    const auto kernel = det ? rk4_tile_kernel<true> : rk4_tile_kernel<false>;
+    const cudaError_t e = allow_smem(allowed[det ? 1 : 0], kernel, smem);
+    if (e != cudaSuccess) return e;
+    return launch_pdl(kernel, dim3(grid), dim3(RK_THREADS), smem, s, a);
 }
 
 }  // namespace tmg

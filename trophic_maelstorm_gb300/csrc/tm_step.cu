@@ -254,21 +254,16 @@ __global__ void __launch_bounds__(256) dornic_deferred_kernel(const DornicArgs<f
 template <int REM, int SAMP, int CAP = kSamplerCap>
 cudaError_t launch_dornic_t(const DornicArgs<float>& a, int grid, int block, size_t smem, cudaStream_t s)
 {
-    static bool attr_set = false;
-    if (!attr_set) {
-        const int full = (int)(warp_scratch_bytes(kMaxRowsPerTask) * kWarps);
-        const cudaError_t e = cudaFuncSetAttribute(dornic_step_kernel<REM, SAMP, CAP>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, full);
-        if (e != cudaSuccess) return e;
-        attr_set = true;
-    }
+    static PerDevice allowed;
+    cudaError_t e = allow_smem(allowed, dornic_step_kernel<REM, SAMP, CAP>, warp_scratch_bytes(kMaxRowsPerTask) * kWarps);
+    if (e != cudaSuccess) return e;
     const int n_seg = grid * (block >> 5);   // one list segment per warp of the step kernel
     // every warp's segment must hold all sites of its tasks
     const long long need = ((long long)a.n_tasks + n_seg - 1) / n_seg * a.rows_cap * 32;
     if (a.dlist == nullptr || a.dcnt == nullptr || need > a.seg_cap || (long long)n_seg > a.max_seg ||
         (long long)n_seg * a.seg_cap > a.dlist_cap)
         return cudaErrorInvalidValue;
-    const cudaError_t e = launch_pdl(dornic_step_kernel<REM, SAMP, CAP>, dim3(grid), dim3(block), smem, s, a);
+    e = launch_pdl(dornic_step_kernel<REM, SAMP, CAP>, dim3(grid), dim3(block), smem, s, a);
     if (e != cudaSuccess) return e;
     return launch_pdl(dornic_deferred_kernel<REM, SAMP, CAP>, dim3((n_seg + 7) / 8), dim3(256), 0, s, a, n_seg);
 }

@@ -644,14 +644,9 @@ namespace {
 template <int REM, int SAMP, int CAP = kSamplerCap>
 cudaError_t launch64_t(const DornicArgs<double>& a, int grid, int block, cudaStream_t s)
 {
-    static bool attr_set = false;
-    if (!attr_set) {
-        const cudaError_t e = cudaFuncSetAttribute(dornic_step64_kernel<REM, SAMP, CAP>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)(warp_bytes(kMaxRowsPerTask) * kWarps));
-        if (e != cudaSuccess) return e;
-        attr_set = true;
-    }
+    static PerDevice allowed;
+    const cudaError_t e = allow_smem(allowed, dornic_step64_kernel<REM, SAMP, CAP>, warp_bytes(kMaxRowsPerTask) * kWarps);
+    if (e != cudaSuccess) return e;
     return launch_pdl(dornic_step64_kernel<REM, SAMP, CAP>, dim3(grid), dim3(block), warp_bytes(a.rows_cap) * kWarps, s, a);
 }
 
