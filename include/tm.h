@@ -186,7 +186,9 @@ int tm_batch_enqueue_steps(tm_batch* b, int64_t n_steps);
  * per SM of the persistent grid.  0 keeps the current value.  A new batch
  * starts at 8 rows (fewer when the batch has too few tasks to fill the GPU) and
  * 4 CTAs/SM.  tm_batch_autotune times the candidates on the batch itself
- * (state is saved and restored).  Results do not depend on the launch shape. */
+ * (state is saved and restored).  Results do not depend on the launch shape.
+ * When memory is short for a shape's tables, tm_batch_set_launch returns
+ * TM_ERR_NOMEM and the batch keeps the shape it had. */
 int tm_batch_set_launch(tm_batch* b, int rows_per_task, int ctas_per_sm);
 int tm_batch_get_launch(const tm_batch* b, int* rows_per_task, int* ctas_per_sm);
 int tm_batch_autotune(tm_batch* b, int steps_per_trial);
@@ -367,12 +369,18 @@ int tm_mlp_predict(tm_mlp* m, const float* x, int n, float* y);
  *   TM_PROBE_MLP_WAIT      the network kernel issues no MMA and waits for a commit
  *                          that never comes: tm_mlp_* return TM_ERR_TIMEOUT and
  *                          leave the parameters unchanged
+ *   TM_PROBE_LIST_GROW     an FP32 batch finds no memory for a longer list of
+ *                          deferred sites than it was created with: a launch
+ *                          shape of more CTAs per SM runs with the CTAs that the
+ *                          list has room for, and one of other rows that needs
+ *                          more is refused (TM_ERR_NOMEM) and changes nothing
  * The flags apply to batches created, and network calls made, after this call
  * on this context (a batch's step graphs keep its launch arguments); 0 clears
  * them.  The context stays usable in every case. */
 #define TM_PROBE_SAMPLER_CAP1 0x1u
 #define TM_PROBE_TILE_WAIT    0x2u
 #define TM_PROBE_MLP_WAIT     0x4u
+#define TM_PROBE_LIST_GROW    0x8u
 int tm_set_test_probe(tm_ctx* ctx, uint32_t flags);
 
 /* Packed-layout geometry without a batch (for callers that pack host buffers

@@ -14,7 +14,7 @@ LIB_PATH = os.path.join(PKG, "lib", "libtm.so")
 TM_OK, TM_ERR_INVALID, TM_ERR_CUDA, TM_ERR_NOMEM, TM_ERR_STATE, TM_ERR_TIMEOUT = 0, -1, -2, -3, -4, -5
 TM_MLP_NPARAMS = 33794
 TM_STATUS_NAN, TM_STATUS_NEGATIVE, TM_STATUS_SAMPLER_CAP, TM_STATUS_WAIT_TIMEOUT = 0x1, 0x2, 0x4, 0x8
-TM_PROBE_SAMPLER_CAP1, TM_PROBE_TILE_WAIT, TM_PROBE_MLP_WAIT = 0x1, 0x2, 0x4
+TM_PROBE_SAMPLER_CAP1, TM_PROBE_TILE_WAIT, TM_PROBE_MLP_WAIT, TM_PROBE_LIST_GROW = 0x1, 0x2, 0x4, 0x8
 TM_FP64, TM_FP32 = 0, 1
 TM_REM_EULER_EXACT, TM_REM_RK4 = 0, 1
 TM_SAMPLER_EXACT, TM_SAMPLER_REF_GAUSS100, TM_SAMPLER_OFF = 0, 1, 2

@@ -68,7 +68,8 @@ struct tm_batch {
     void* aux = nullptr;        // Rietkerk P* (field-0 slots)
     uint4* d_dlist = nullptr;   // FP32: sites the straight-line draw deferred, a segment per warp of the grid
     unsigned* d_dcnt = nullptr;
-    long long dlist_cap = 0, max_seg = 0;
+    long long dlist_cap = 0, dcnt_cap = 0;   // allocated: entries, segments
+    long long max_seg = 0;                   // segments that the launch may use
     void* site_b = nullptr;     // per-site loss coefficient (DP), packed like the state
     long long* d_step = nullptr;
     int64_t step = 0;
@@ -181,17 +182,72 @@ int rk64_tile_rows(const tm_batch* b)
 }
 
 // Warps of the FP32 step's grid at most, each with a segment of the deferred-site list.
-long long list_segments(const tm_batch* b)
+long long list_segments(const tm_batch* b, long long n_tasks, int ctas)
 {
-    return std::min<long long>((long long)b->n_tasks + 8, (long long)std::max(1, b->ctx->num_sms) * std::max(b->ctas_per_sm, 4) * 8);
+    return std::min<long long>(n_tasks + 8, (long long)std::max(1, b->ctx->num_sms) * std::max(ctas, 4) * 8);
 }
 
-int build_tasks(tm_batch* b)
+// Room for a deferred-site list of `entries` in `segs` segments.  False when memory is
+// short; the list is then what it was (if even that cannot be had again it is empty, and
+// every launch is refused on the host).  Its addresses may have changed either way.
+bool grow_list(tm_batch* b, long long entries, long long segs)
+{
+    if (entries <= b->dlist_cap && segs <= b->dcnt_cap) return true;
+    uint4* list = nullptr;
+    unsigned* cnt = nullptr;
+    const auto get = [&](long long n, long long m) {
+        const bool refuse = (b->probe & TM_PROBE_LIST_GROW) && b->max_seg > 0 && (n > b->dlist_cap || m > b->dcnt_cap);
+        if (!refuse && cuda_ok(dalloc(&list, (size_t)n)) && cuda_ok(dalloc(&cnt, (size_t)m))) return true;
+        cudaFree(list);
+        list = nullptr;
+        (void)cudaGetLastError();
+        return false;
+    };
+    const auto install = [&](long long n, long long m) {
+        cudaFree(b->d_dlist);
+        cudaFree(b->d_dcnt);
+        b->d_dlist = list;
+        b->d_dcnt = cnt;
+        b->dlist_cap = n;
+        b->dcnt_cap = m;
+    };
+    if (get(entries, segs)) {
+        install(entries, segs);
+        return true;
+    }
+    if (!b->d_dlist) return false;
+    // perhaps the old and the new one only do not fit together
+    const long long had = b->dlist_cap, had_segs = b->dcnt_cap;
+    cudaFree(b->d_dlist); b->d_dlist = nullptr;
+    cudaFree(b->d_dcnt); b->d_dcnt = nullptr;
+    if (get(entries, segs)) {
+        install(entries, segs);
+        return true;
+    }
+    if (get(had, had_segs)) install(had, had_segs);
+    else b->dlist_cap = b->dcnt_cap = b->max_seg = 0;
+    return false;
+}
+
+// The deferred-site list for n_tasks tasks of R rows: a step grid of nw warps gives every
+// warp a segment of ceil(n_tasks / nw) tasks' sites, nw * that <= (n_tasks + nw) * R * 32
+// entries; sized for a grid of `ctas` blocks per SM (the default's at least), at most one
+// warp per task.
+bool fit_list(tm_batch* b, long long n_tasks, int R, int ctas)
+{
+    const long long segs = list_segments(b, n_tasks, ctas);
+    if (!grow_list(b, (n_tasks + segs) * R * 32, segs)) return false;
+    b->max_seg = segs;
+    return true;
+}
+
+// Task tables for R rows per task.  On an error the batch keeps the tables and the launch
+// that it had.
+int build_tasks(tm_batch* b, int R)
 {
     // warp tasks
     std::vector<int4> tasks;
     std::vector<int> begin(b->n_inst + 1, 0);
-    const int R = b->rows_per_task;
     tasks.reserve((size_t)count_tasks(b, R));
     for (int k = 0; k < b->n_inst; ++k) {
         begin[k] = (int)tasks.size();
@@ -201,19 +257,26 @@ int build_tasks(tm_batch* b)
     }
     begin[b->n_inst] = (int)tasks.size();
     if (tasks.size() > (size_t)0x7fffffff) return TM_ERR_INVALID;
-    cudaFree(b->d_tasks); b->d_tasks = nullptr;
-    cudaFree(b->d_partial); b->d_partial = nullptr;
-    b->n_tasks = (int)tasks.size();
-    TM_CUDA(dalloc(&b->d_tasks, tasks.size()));
     // partials and group sums, four numbers each; the arrival counters follow the table of
     // first tasks, whose upload sets them to 0
-    b->n_groups = measure_group_base(b->n_tasks, b->n_inst) + 1;
-    TM_CUDA(dalloc(&b->d_partial, 4 * (tasks.size() + b->n_groups)));
-    begin.resize((size_t)b->n_inst + 1 + b->n_inst + b->n_groups, 0);
-    TM_CUDA(cudaMemcpy(b->d_tasks, tasks.data(), tasks.size() * sizeof(int4), cudaMemcpyHostToDevice));
-    cudaFree(b->d_task_begin); b->d_task_begin = nullptr;
-    TM_CUDA(dalloc(&b->d_task_begin, begin.size()));
-    TM_CUDA(cudaMemcpy(b->d_task_begin, begin.data(), begin.size() * sizeof(int), cudaMemcpyHostToDevice));
+    const int n_groups = measure_group_base((int)tasks.size(), b->n_inst) + 1;
+    begin.resize((size_t)b->n_inst + 1 + b->n_inst + n_groups, 0);
+    int4* d_tasks = nullptr;
+    double* d_partial = nullptr;
+    int* d_begin = nullptr;
+    const auto drop = [&](int rc) {
+        cudaFree(d_tasks);
+        cudaFree(d_partial);
+        cudaFree(d_begin);
+        (void)cudaGetLastError();
+        return rc;
+    };
+    if (!cuda_ok(dalloc(&d_tasks, tasks.size())) || !cuda_ok(dalloc(&d_partial, 4 * (tasks.size() + n_groups))) ||
+        !cuda_ok(dalloc(&d_begin, begin.size())))
+        return drop(TM_ERR_NOMEM);
+    if (!cuda_ok(cudaMemcpy(d_tasks, tasks.data(), tasks.size() * sizeof(int4), cudaMemcpyHostToDevice)) ||
+        !cuda_ok(cudaMemcpy(d_begin, begin.data(), begin.size() * sizeof(int), cudaMemcpyHostToDevice)))
+        return drop(TM_ERR_CUDA);
     // 64 x 32 tiles (Rietkerk RK4, noise-off DP; FP64 Rietkerk: rk64_tile_rows)
     if ((b->model == 1 || b->dpm.deterministic) && !b->d_btasks) {
         std::vector<int4> bt;
@@ -223,23 +286,23 @@ int build_tasks(tm_batch* b)
             for (int y0 = 0; y0 < L; y0 += ty)
                 for (int x0 = 0; x0 < L; x0 += RK_TX) bt.push_back(make_int4(k, x0, y0, ty));
         }
+        if (!cuda_ok(dalloc(&b->d_btasks, bt.size()))) return drop(TM_ERR_NOMEM);
+        if (!cuda_ok(cudaMemcpy(b->d_btasks, bt.data(), bt.size() * sizeof(int4), cudaMemcpyHostToDevice)))
+            return drop(TM_ERR_CUDA);
         b->n_btasks = (int)bt.size();
-        TM_CUDA(dalloc(&b->d_btasks, bt.size()));
-        TM_CUDA(cudaMemcpy(b->d_btasks, bt.data(), bt.size() * sizeof(int4), cudaMemcpyHostToDevice));
-    }
-    if (b->precision == TM_FP32) {
-        // the deferred-site list: a step grid of nw warps gives every warp a segment of
-        // ceil(n_tasks / nw) tasks' sites, nw * that <= (n_tasks + nw) * R * 32 entries; sized
-        // for the grid of ctas_per_sm (the default's at least), at most one warp per task
-        cudaFree(b->d_dlist); b->d_dlist = nullptr;
-        cudaFree(b->d_dcnt); b->d_dcnt = nullptr;
-        b->max_seg = list_segments(b);
-        b->dlist_cap = ((long long)b->n_tasks + b->max_seg) * R * 32;
-        TM_CUDA(dalloc(&b->d_dlist, (size_t)b->dlist_cap));
-        TM_CUDA(dalloc(&b->d_dcnt, (size_t)b->max_seg));
     }
     free_graphs(b);
-    return TM_OK;
+    // a list for fewer blocks per SM holds the grid down to what it has segments for
+    if (b->precision == TM_FP32 && !fit_list(b, (long long)tasks.size(), R, b->ctas_per_sm) &&
+        !fit_list(b, (long long)tasks.size(), R, 0))
+        return drop(TM_ERR_NOMEM);
+    std::swap(b->d_tasks, d_tasks);
+    std::swap(b->d_partial, d_partial);
+    std::swap(b->d_task_begin, d_begin);
+    b->n_tasks = (int)tasks.size();
+    b->n_groups = n_groups;
+    b->rows_per_task = R;
+    return drop(TM_OK);
 }
 
 // Grid of the FP64 step: the resident CTAs (two per SM), or one CTA per task where
@@ -253,7 +316,9 @@ int warp_grid(const tm_batch* b, int n_tasks)
 {
     const int warps_per_cta = 8;
     const int need = (n_tasks + warps_per_cta - 1) / warps_per_cta;
-    const int cap = std::max(1, b->ctx->num_sms * b->ctas_per_sm);
+    int cap = std::max(1, b->ctx->num_sms * b->ctas_per_sm);
+    // FP32: no more warps than the deferred-site list has segments
+    if (b->precision == TM_FP32) cap = (int)std::min<long long>(cap, std::max<long long>(1, b->max_seg / warps_per_cta));
     return std::max(1, std::min(need, cap));
 }
 
@@ -497,8 +562,7 @@ int batch_common_init(tm_batch* b, const tm_instance* inst, int n)
     TM_CUDA(cudaMemset(b->d_step, 0, sizeof(long long)));
 
     b->probe = b->ctx->probe;
-    b->rows_per_task = default_rows(b);
-    return build_tasks(b);
+    return build_tasks(b, default_rows(b));
 }
 
 int obs_reserve(tm_batch* b, int n_meas)
@@ -580,7 +644,7 @@ void* tm_stream(tm_ctx* c) { return c ? (void*)c->stream : nullptr; }
 
 int tm_set_test_probe(tm_ctx* c, uint32_t flags)
 {
-    if (!c || (flags & ~(TM_PROBE_SAMPLER_CAP1 | TM_PROBE_TILE_WAIT | TM_PROBE_MLP_WAIT))) return TM_ERR_INVALID;
+    if (!c || (flags & ~(TM_PROBE_SAMPLER_CAP1 | TM_PROBE_TILE_WAIT | TM_PROBE_MLP_WAIT | TM_PROBE_LIST_GROW))) return TM_ERR_INVALID;
     c->probe = flags;
     return TM_OK;
 }
@@ -865,14 +929,22 @@ int tm_batch_set_launch(tm_batch* b, int rows, int ctas)
     if (!b || rows < 0 || ctas < 0 || rows > kMaxRowsPerTask || ctas > 64) return TM_ERR_INVALID;
     TM_CUDA(cudaSetDevice(b->ctx->device));
     TM_CUDA(cudaStreamSynchronize(b->ctx->stream));
-    bool rebuild = false;
-    if (rows > 0 && rows != b->rows_per_task) { b->rows_per_task = rows; rebuild = true; }
-    if (ctas > 0 && ctas != b->ctas_per_sm) {
+    const int before = b->ctas_per_sm;
+    if (ctas > 0 && ctas != before) {
         b->ctas_per_sm = ctas;
         free_graphs(b);
-        if (b->precision == TM_FP32 && list_segments(b) > b->max_seg) rebuild = true;
     }
-    return rebuild ? build_tasks(b) : TM_OK;
+    if (rows > 0 && rows != b->rows_per_task) {
+        const int rc = build_tasks(b, rows);
+        if (rc != TM_OK) b->ctas_per_sm = before;
+        return rc;
+    }
+    // more blocks per SM want a longer list; without memory for it the present one serves
+    // a grid of as many warps as it has segments
+    if (b->precision == TM_FP32 && list_segments(b, b->n_tasks, b->ctas_per_sm) > b->max_seg &&
+        !fit_list(b, b->n_tasks, b->rows_per_task, b->ctas_per_sm) && !b->d_dlist)
+        return TM_ERR_NOMEM;
+    return TM_OK;
 }
 
 int tm_batch_get_launch(const tm_batch* b, int* rows, int* ctas)
