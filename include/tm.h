@@ -184,8 +184,9 @@ int tm_batch_enqueue_steps(tm_batch* b, int64_t n_steps);
 
 /* Launch shape of the step kernels: rows per warp task (DP/Dornic) and CTAs
  * per SM of the persistent grid.  0 keeps the current value.  A new batch
- * starts at 8 rows (fewer when the batch has too few tasks to fill the GPU) and
- * 4 CTAs/SM.  tm_batch_autotune times the candidates on the batch itself
+ * starts at 8 rows (fewer when the batch has too few tasks to fill the GPU, 16
+ * for a large FP32 DP batch) and as many CTAs per SM as are resident: 4 in FP32,
+ * 2 in FP64.  tm_batch_autotune times the candidates on the batch itself
  * (state is saved and restored).  Results do not depend on the launch shape.
  * When memory is short for a shape's tables, tm_batch_set_launch returns
  * TM_ERR_NOMEM and the batch keeps the shape it had. */

@@ -305,18 +305,22 @@ int build_tasks(tm_batch* b, int R)
     return drop(TM_OK);
 }
 
-// Grid of the FP64 step: the resident CTAs (two per SM), or one CTA per task where
-// there are fewer -- its warps take tasks from different parts of the list.
+// CTAs per SM of a new batch's step: the resident ones.
+int default_ctas(const tm_batch* b) { return b->precision == TM_FP64 ? 2 : 4; }
+
+// Grid of the FP64 step: ctas_per_sm per SM, or one CTA per task where there are fewer --
+// its warps take tasks from different parts of the list.
 int step64_grid(const tm_batch* b)
 {
-    return std::max(1, std::min(b->n_tasks, b->ctx->num_sms * std::min(b->ctas_per_sm, 2)));
+    return std::max(1, std::min(b->n_tasks, b->ctx->num_sms * b->ctas_per_sm));
 }
 
 int warp_grid(const tm_batch* b, int n_tasks)
 {
     const int warps_per_cta = 8;
     const int need = (n_tasks + warps_per_cta - 1) / warps_per_cta;
-    int cap = std::max(1, b->ctx->num_sms * b->ctas_per_sm);
+    // FP64: measurements, whose kernels have more CTAs resident than the step
+    int cap = std::max(1, b->ctx->num_sms * std::max(b->ctas_per_sm, b->precision == TM_FP64 ? 4 : 1));
     // FP32: no more warps than the deferred-site list has segments
     if (b->precision == TM_FP32) cap = (int)std::min<long long>(cap, std::max<long long>(1, b->max_seg / warps_per_cta));
     return std::max(1, std::min(need, cap));
@@ -562,6 +566,7 @@ int batch_common_init(tm_batch* b, const tm_instance* inst, int n)
     TM_CUDA(cudaMemset(b->d_step, 0, sizeof(long long)));
 
     b->probe = b->ctx->probe;
+    b->ctas_per_sm = default_ctas(b);
     return build_tasks(b, default_rows(b));
 }
 
