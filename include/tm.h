@@ -272,9 +272,17 @@ int tm_observe_noalloc(const void* dev_fields, int precision, const int32_t* L, 
  * L / kvals[argmax power].  Synchronises `stream`. */
 int tm_power_spectrum_device(const void* dev_field, int precision, int L, double binwidth, void* stream,
                              double* kvals, double* power, int max_bins, int* n_bins);
-/* The same for field `field` of instance k of a batch's current state. */
+/* The same for field `field` of instance k of a batch's current state.  The batch
+ * keeps the transform's plan and buffers (16 L^2 bytes and the transform's own
+ * work area) for its next call of the same side and bin width, until a call of
+ * another side or width replaces them, tm_batch_release_work gives them back,
+ * or the batch is destroyed. */
 int tm_batch_power_spectrum(tm_batch* b, int k, int field, double binwidth, double* kvals, double* power,
                             int max_bins, int* n_bins);
+/* Frees the device memory that a batch keeps between calls beyond its state and
+ * tables (the plan and buffers of tm_batch_power_spectrum); the next call that
+ * needs it allocates it again. */
+int tm_batch_release_work(tm_batch* b);
 
 /* -- consumer movement: FKE advection-diffusion ---------------------------
  * Replaces advdiff_FKE_MultiSp (simulations/Rietkerk_FPE/rietkerk_bjork_FKE.cpp:

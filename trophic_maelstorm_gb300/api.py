@@ -281,7 +281,8 @@ class Batch:
 
     def power_spectrum(self, k, field=0, binwidth=0.5):
         """Radially averaged power spectrum of instance k's field (glow_up.py:752-827
-        semantics); returns (kvals, power)."""
+        semantics); returns (kvals, power).  The batch keeps the transform's plan and
+        buffers for its next call (release_work frees them)."""
         L = self.inst[k].L
         cap = int(2 * L / binwidth) + 8
         kv = np.zeros(cap)
@@ -291,6 +292,10 @@ class Batch:
                                                 pw.ctypes.data_as(C.POINTER(C.c_double)), cap, C.byref(nb)),
                 "tm_batch_power_spectrum")
         return kv[:nb.value], pw[:nb.value]
+
+    def release_work(self):
+        """Free the device memory kept between calls beyond state and tables."""
+        T.check(T.lib().tm_batch_release_work(self._h), "tm_batch_release_work")
 
     def close(self):
         if self._h:

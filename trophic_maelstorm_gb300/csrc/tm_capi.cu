@@ -1099,6 +1099,16 @@ int tm_batch_power_spectrum(tm_batch* b, int k, int field, double binwidth, doub
                           &b->spectrum);
 }
 
+int tm_batch_release_work(tm_batch* b)
+{
+    if (!b) return TM_ERR_INVALID;
+    TM_CUDA(cudaSetDevice(b->ctx->device));
+    TM_CUDA(cudaStreamSynchronize(b->ctx->stream));
+    spectrum_work_destroy(b->spectrum);
+    b->spectrum = nullptr;
+    return TM_OK;
+}
+
 static int run_common(tm_batch* b, const void* init, int64_t n_steps, const int64_t* meas, int n_meas, double* obs,
                       uint32_t* status, void* fin)
 {
