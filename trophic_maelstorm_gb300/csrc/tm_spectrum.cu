@@ -132,14 +132,21 @@ struct Annuli {
     std::vector<long long> lim;
 };
 
+// Their number without listing them; more than an int holds counts as the largest int.
+int count_annuli(int L, double bw)
+{
+    const double start = 1.0 - bw / 2.0, stop = (double)(L / 2 + 1);
+    const double n = std::ceil((stop - start) / bw) - 1.0;    // numpy.arange's length, less one
+    return n >= 1.0 ? (n < 2147483647.0 ? (int)n : 2147483647) : 0;
+}
+
 void make_annuli(int L, double bw, Annuli& p)
 {
     // edges: numpy.arange(1 - bw/2, L//2 + 1, bw)
-    std::vector<double> e;
-    const double start = 1.0 - bw / 2.0, stop = (double)(L / 2 + 1);
-    const long long ne = (long long)std::ceil((stop - start) / bw);
-    for (long long i = 0; i < ne; ++i) e.push_back(start + (double)i * bw);
-    p.nbins = e.size() > 1 ? (int)e.size() - 1 : 0;
+    p.nbins = count_annuli(L, bw);
+    std::vector<double> e(p.nbins ? (size_t)p.nbins + 1 : 0);
+    const double start = 1.0 - bw / 2.0;
+    for (size_t i = 0; i < e.size(); ++i) e[i] = start + (double)i * bw;
     p.kvals.resize(p.nbins);
     p.area.resize(p.nbins);
     for (int b = 0; b < p.nbins; ++b) {
@@ -187,10 +194,9 @@ struct SpectrumWork {
         (void)cudaGetLastError();
     }
 
-    // Plan and buffers (nothing of them when the lattice has no annulus).
+    // Plan and buffers.
     int prepare(cudaStream_t s)
     {
-        if (ann.nbins == 0) return TM_OK;
         const size_t n = (size_t)L * L;
         SPEC_CUDA(cudaMalloc(&img, n * sizeof(double)));
         SPEC_CUDA(cudaMalloc(&F, (size_t)L * (L / 2 + 1) * sizeof(cufftDoubleComplex)));
@@ -235,16 +241,18 @@ int power_spectrum(const void* dev_field, int precision, int L, double binwidth,
     if (precision != TM_FP64 && precision != TM_FP32) return TM_ERR_INVALID;
     SpectrumWork* w = keep ? *keep : nullptr;
     if (!w || w->L != L || w->bw != binwidth) {
+        *n_bins = count_annuli(L, binwidth);
+        if (*n_bins > max_bins) return TM_ERR_INVALID;
+        if (*n_bins == 0) return TM_OK;
         SpectrumWork* fresh = new (std::nothrow) SpectrumWork;
         if (!fresh) return TM_ERR_NOMEM;
         fresh->L = L;
         fresh->bw = binwidth;
-        make_annuli(L, binwidth, fresh->ann);
-        *n_bins = fresh->ann.nbins;
-        if (fresh->ann.nbins > max_bins || fresh->ann.nbins == 0) {
-            const int rc = fresh->ann.nbins > max_bins ? TM_ERR_INVALID : TM_OK;
+        try {
+            make_annuli(L, binwidth, fresh->ann);
+        } catch (const std::bad_alloc&) {
             delete fresh;
-            return rc;
+            return TM_ERR_NOMEM;
         }
         if (keep) {
             delete w;                       // first, so that both never hold memory together
