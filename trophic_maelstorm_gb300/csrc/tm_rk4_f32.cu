@@ -12,10 +12,8 @@
 //
 // A thread evaluates two neighbouring cells at once with 8-byte shared-memory accesses.
 // The region is 36 pairs wide; pairs that stick out of a stage's inset compute a cell
-// nobody reads.  The reciprocals are the FP32 estimate and one fused Newton step, which
-// rounds correctly when the estimate is within an ulp (Markstein 1990; compared with
-// __frcp_rn for every mantissa: no difference); a pair whose residuals show an argument
-// outside that method's range takes __frcp_rn.
+// nobody reads.  The reciprocals are the FP32 estimate and one fused Newton step (neg_rcp);
+// a pair whose residuals show an argument outside that method's range takes __frcp_rn.
 // Measured at 2048^2: 83.5 us a step one cell at a time with __frcp_rn and every warp
 // polling for the copies, 73 us now; bound by the stages' barriers and the issue slots
 // (58 %) in turns.  Slower: three CTAs of 64 x 20 tiles (2 %), four of 64 x 12 (4 %), one
@@ -43,16 +41,6 @@
 namespace tmg {
 
 namespace {
-
-// -1/x; ok stays true only while the method holds (see above)
-__device__ __forceinline__ float neg_rcp(float x, bool& ok)
-{
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(-x));
-    const float e = fmaf(x, r, 1.0f);
-    ok = ok && fabsf(e) < 0x1p-20f;
-    return fmaf(r, e, r);
-}
 
 __device__ __forceinline__ float2 ld2(const float* p) { return *reinterpret_cast<const float2*>(p); }
 
