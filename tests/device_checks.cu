@@ -206,6 +206,26 @@ __global__ void k_open_unit(Result* r, unsigned long long, unsigned long long)
     note(r, n, bad, 0, 0);
 }
 
+// unit_f32 against the FP64 uniform of the same words and of their complements; worst is
+// the largest relative difference in units of 2^-23
+__global__ void k_unit(Result* r, unsigned long long n_words, unsigned long long)
+{
+    unsigned long long n = 0, bad = 0;
+    float worst = 0.0f;
+    for (unsigned long long i = index0(); i < n_words; i += stride(), ++n) {
+        const unsigned long long h = mix(i);
+        // leading words 0 to 7, all ones, and of every length
+        const uint32_t w1 = i < (1u << 20) ? (uint32_t)(i & 7) : (i < (2u << 20) ? ~(uint32_t)(i & 7) : (uint32_t)(h >> 32) >> (i & 31));
+        const uint32_t w2 = (i & 64) ? (uint32_t)h >> ((h >> 40) & 31) : (uint32_t)h;
+        const double u = tmf::open_unit(((unsigned long long)w1 << 21) | (w2 >> 11));
+        const float share = (float)(fabs((double)unit_f32(w1, w2) - u) / u * 0x1p23);
+        worst = fmaxf(worst, share);
+        bad += !(share <= 1.0f + 0x1p-20f);
+    }
+    note(r, n, bad, 0, 0);
+    atomicMax(&r->worst, __float_as_uint(worst));
+}
+
 // ---- decisions in FP32 against the FP64 method
 __device__ double mean_below_32(unsigned long long h)
 {
@@ -342,6 +362,7 @@ CHECK(f64, k_f64)
 CHECK(recip31, k_recip31)
 CHECK(f64_sqrt, k_sqrt)
 CHECK(open_unit, k_open_unit)
+CHECK(unit, k_unit)
 CHECK(search, k_search)
 CHECK(search_tails, k_search_tails)
 CHECK(ptrs, k_ptrs<kSamplerCap>)

@@ -78,3 +78,7 @@ def test_poisson_search(checks):
 @pytest.mark.parametrize("name", ["ptrs", "ptrs_cap", "normal", "normal_cap", "gamma", "gamma_cap"])
 def test_draws_match_the_fp64_methods(checks, name):
     assert checks(name, 1 << 26).n == 1 << 26
+
+
+def test_fp32_uniform(checks):
+    assert checks("unit", 1 << 26).worst > 0

@@ -66,22 +66,38 @@ __device__ __forceinline__ int search_count(bool need, float m, uint32_t w, cons
     return run ? -1 : n;
 }
 
-// FP32 value of a uniform from its two words, relative error 2^-22
+// FP32 value of the uniform that Stream<double>::open forms of two words, (x + 1/2) 2^-53
+// with x the 53 leading bits: within 2^-23 relative, whatever the words (the roundings of
+// w1 and of the sum; the low part is exact).
 __device__ __forceinline__ float unit_f32(uint32_t w1, uint32_t w2)
 {
-    return fmaf((float)w1, 0x1p-32f, (float)((w2 >> 11) + 1u) * 0x1p-53f);
+    return fmaf((float)w1, 0x1p-32f, ((float)(w2 >> 11) + 0.5f) * 0x1p-53f);
 }
 
 // poisson_exact for m >= 32 (PTRS) with its floor and its tests decided in FP32 where the
 // error bounds allow: the candidate k is taken when the FP32 value lies further from a
-// whole number than its error (relative 2^-20 of the terms' sizes, a handful of roundings
-// of 2^-24 each), a comparison when the two sides differ by more than theirs (the logs'
-// arguments are good to 2^-21, k log1p((k + 1 - m) / m) to m 2^-24 besides its own size).
+// whole number than its error, a comparison when the two sides differ by more than theirs.
 // Anything closer runs the FP64 method from the same counter; beyond 4096 that would be
 // most draws.  The FP64 method is six divisions, a root and up to six logs on a pipe that
 // takes a warp instruction every 64 cycles: with it the list of general draws was 30 % of
 // the whole kernel on a Rietkerk run (means up to 100); 16 lattices of 256^2, 20 steps:
 // 9.24 ms before, 8.79 ms with this.
+//
+// The errors, in units of e = 2^-24 (one rounding); a log's is |log| + 3:
+//   mf 1 m;  slam 1.5 slam;  b 4.5 b;  a 9 a (its terms cancel by 1.19 at b = 15);
+//   us 2 us (unit_f32), U 2;  2 a / us 12, scale 13 scale;  scale U 9 scale (|U| <= 1/2)
+//   x: 9 scale + m, and the two sums' scale + 2 m + 1: 10 scale + 3 m + 1, where err is
+//     16 scale + 32 m + 32 (so us below 2^-19, where scale passes 2^19, is never sure)
+//   us and V against 0.07, vr and 0.013: 2 of each and 30 for vr (3.6 / (b - 2) at b = 15),
+//     where the bands are 1e-4, 1e-5 and 1e-6, 16 at least
+//   lhs: log V 2 + |log V| + 3;  loginvalpha 7;  log(a / us^2 + b) 17 + |log| + 3;  the two
+//     sums |lhs| each: below 33 + 3 |lhs|, as |log V| and the last log add up to |lhs| + 0.2
+//   rhs, k < 16: k (log m + 4) + 4 (k log m + m + log k!): below 60 + 5 size
+//   rhs, else: an error of m or d moves d - k log1p(d/m) by itself times |k - m|/m or 1/z
+//     only; the quotient |d|, the log1p 15 |kl| (below -0.29 and above 0.41: the rounding
+//     of 1 + x and the log's, where |l| > 0.34; else 4 |kl|), the product and the sums |kl| +
+//     2 |d| + |log z| + 4, the dropped term of corr 6e-10: below 16 |kl| + 3 |d| + 20
+//   tol is 32 (size + m/4 + |lhs| + 16) + 67: twice their sum or more.
 template <int CAP>
 __device__ __forceinline__ double ptrs64(Stream<double>& g, double m, const Tab64& tb)
 {
