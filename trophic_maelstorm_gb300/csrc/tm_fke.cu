@@ -329,9 +329,10 @@ __global__ void __launch_bounds__(kCols) fke_cols_kernel(const T* __restrict__ A
     if (p0 + 1 < L) out[(p0 + 1) * L + q] = a1;
 }
 
-// Workspace of one call (each region 256-byte aligned): w, A_D, A_V (T, L^2 each),
-// the landing sites and a spare region of the same size (4 bytes, L^2 each), the wrapped
-// stencils gDw, gVw (T, L each), smax (int).
+// Workspace of one call (each region 256-byte aligned): w, A_D, A_V (T, L^2 each), the
+// landing sites (4 bytes, L^2), a region of the same size that is not used -- callers
+// allocate by the size tm_fke_workspace_bytes has always given -- the wrapped stencils gDw,
+// gVw (T, L each), smax (int).
 struct FkeLayout {
     size_t w, AD, AV, to, spare, gD, gV, smax, end;
 };

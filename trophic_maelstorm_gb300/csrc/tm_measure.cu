@@ -12,8 +12,9 @@
 // A measurement is short beside its launches and round trips.  With a second kernel of
 // one warp per instance for the sums, 64 spreading FP64 lattices of 101 x 101 took 18.7 us
 // to measure, 12.8 us with the sums in the same launch (and no additions for rows of
-// zeros), 8.6 us with one-field code of its own (64 registers instead of 102); on a 4096 x 4096 FP32 Rietkerk lattice that one warp walked 65,536 partials, 613
-// us of a run of 24 steps and one measurement that went from 12.31 to 11.75 ms.
+// zeros), 8.6 us with one-field code of its own (64 registers instead of 102); on a 4096 x
+// 4096 FP32 Rietkerk lattice that one warp walked 65,536 partials, 613 us of a run of 24
+// steps and one measurement that went from 12.31 to 11.75 ms.
 //
 // GB300's FP64 rate is a small fraction of its FP32 rate, so the per-site work
 // avoids FP64: active sites are counted with ballots, and an FP32 lane keeps
